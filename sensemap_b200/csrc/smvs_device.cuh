@@ -78,7 +78,7 @@ __device__ inline void CorrectNormal(float n[3], const float vd[3], float inv_vi
     float c3[3];
     c3[0] = n[1] * vd[2] - n[2] * vd[1];
     c3[1] = n[2] * vd[0] - n[0] * vd[2];
-    c3[2] = n[0] * vd[1] - n[1] * vd[0];
+    c3[2] = __fmaf_rn(n[0], vd[1], -__fmul_rn(n[1], vd[0]));
     float phi = (float)((double)acosf(cal * inv_view_len) - 90.0 * 0.0174532925199432);
     phi = fminf(phi * 1.01f, -0.001f);
     if (phi == 0) return;
@@ -101,9 +101,9 @@ __device__ inline void CorrectNormal(float n[3], const float vd[3], float inv_vi
     Rt[0] = 1 + om[0] * sp + cO[0]; Rt[1] = 0 + om[1] * sp + cO[1]; Rt[2] = 0 + om[2] * sp + cO[2];
     Rt[3] = 0 + om[3] * sp + cO[3]; Rt[4] = 1 + om[4] * sp + cO[4]; Rt[5] = 0 + om[5] * sp + cO[5];
     Rt[6] = 0 + om[6] * sp + cO[6]; Rt[7] = 0 + om[7] * sp + cO[7]; Rt[8] = 1 + om[8] * sp + cO[8];
-    const float r0 = Rt[0] * n[0] + Rt[1] * n[1] + Rt[2] * n[2];
-    const float r1 = Rt[3] * n[0] + Rt[4] * n[1] + Rt[5] * n[2];
-    const float r2 = Rt[6] * n[0] + Rt[7] * n[1] + Rt[8] * n[2];
+    const float r0 = __fmaf_rn(Rt[2], n[2], __fmaf_rn(Rt[0], n[0], __fmul_rn(Rt[1], n[1])));
+    const float r1 = __fmaf_rn(Rt[5], n[2], __fmaf_rn(Rt[3], n[0], __fmul_rn(Rt[4], n[1])));
+    const float r2 = __fmaf_rn(Rt[8], n[2], __fmaf_rn(Rt[6], n[0], __fmul_rn(Rt[7], n[1])));
     n[0] = r0; n[1] = r1; n[2] = r2;
   }
 }
@@ -113,8 +113,9 @@ __device__ __forceinline__ float PropagateDepth(float d1, const float n1[3], con
                                                 int col1, const float p2[3]) {
   const float x1 = d1 * (iK[0] * col1 + iK[1]);
   const float y1 = d1 * (iK[2] * row1 + iK[3]);
-  const float d = n1[0] * x1 + n1[1] * y1 + n1[2] * d1;
-  const float t = d / (n1[0] * p2[0] + n1[1] * p2[1] + n1[2] * p2[2]);
+  const float d = __fmaf_rn(n1[2], d1, __fmaf_rn(n1[0], x1, __fmul_rn(n1[1], y1)));
+  const float q = __fadd_rn(__fmaf_rn(n1[1], p2[1], __fmul_rn(n1[0], p2[0])), n1[2]);  // p2[2] = 1
+  const float t = d / q;
   if (fabsf(t) < 1e-5f) return d1;
   return t;
 }
@@ -122,7 +123,7 @@ __device__ __forceinline__ float PropagateDepth(float d1, const float n1[3], con
 // PerturbNormal (ACMH form) via Normal2Dir / Dir2Normal: kernel_functions.cu:214-225,
 // utils.h:94-106.
 __device__ __forceinline__ void PerturbNormalACMH(const float n[3], float out[3], float a1, float a2, Rng& r) {
-  const float y = atan2f(sqrtf(n[0] * n[0] + n[1] * n[1]), n[2]);
+  const float y = atan2f(sqrtf(__fmaf_rn(n[0], n[0], __fmul_rn(n[1], n[1]))), n[2]);
   const float x = atan2f(n[1], n[0]);
   const float nx = a1 * (2 * r.Uniform() - 1) + x;
   const float ny = a2 * (2 * r.Uniform() - 1) + y;

@@ -351,6 +351,12 @@ __device__ __forceinline__ float ViewCost(const JobParams& p, const float* poses
   return cost;
 }
 
+// Whether a partial sum of a hypothesis's weighted costs proves it worse than
+// `best`: costs and weights are not negative, so the full sum is at least the
+// partial one, and the margin is above the rounding of either sum (at most 32
+// terms). A NaN compares false and proves nothing.
+__device__ __forceinline__ bool WorseThan(float partial, float best) { return partial > best * 1.00001f; }
+
 // InitConfMapKernel, kernel_functions.cu:1497-1601. One thread per
 // pixel; the cost vector and its sort order live in shared memory
 // ([view][pixel], nb views per pixel).
@@ -556,12 +562,31 @@ __device__ __forceinline__ bool SweepTileL(const Batch& b, int colour, int bid, 
   float costs[kMaxHyp];
   // Two evaluation phases share one call site of the cost code: phase 0 scores
   // the propagated hypotheses 1..ns-1, phase 1 the refinement hypotheses 1..4.
+  // A refinement hypothesis only matters if it beats the pixel's best: once the
+  // views scored so far prove that it does not, its other views are not sampled
+  // (FLT_MAX in their place keeps it from winning). The texture unit bounds this
+  // kernel and serves quads of lanes, so lanes that stop save time even where
+  // others of the warp go on. Measured (1600x1200, 10 views, f16, six
+  // iterations): 17.51 -> 14.76 ms per launch at step 1, 5.85 -> 5.23 at step 2.
   int h_end = ns;
+  float best = FLT_MAX;
   for (int phase = 0; phase < 2; ++phase) {
     for (int h = 1; h < h_end; ++h) {
       const float pw = PriorWeight(p, pri, hyp[h], hyp[h][3], pr.rvar);
-      for (int v = 0; v < N; ++v)
-        M[h][v] = ViewCost<R, S, 1>(p, poses, v, row, col, hyp[h][3], hyp[h], vd, pr, p.refK, 0, gmask, pw);
+      float sum = 0.f;
+      bool out = false;
+      for (int v = 0; v < N; ++v) {
+        float cost = FLT_MAX;
+        if (!out) {
+          cost = ViewCost<R, S, 1>(p, poses, v, row, col, hyp[h][3], hyp[h], vd, pr, p.refK, 0, gmask, pw);
+          if (phase == 1) {
+            sum += vw[v] * cost;
+            out = WorseThan(sum, best);
+          }
+        }
+        M[h][v] = cost;
+      }
+      if (phase == 1 && !out) best = fminf(best, sum);
     }
     if (phase == 1) break;
 
@@ -626,6 +651,7 @@ __device__ __forceinline__ bool SweepTileL(const Batch& b, int colour, int bid, 
         if (costs[h] <= m) { m = costs[h]; mi = h; }  // FindMinCost :648-659 ('<=')
     }
     if (mi < 0) return true;
+    best = costs[mi];
     depth = hyp[mi][3];
     normal[0] = hyp[mi][0]; normal[1] = hyp[mi][1]; normal[2] = hyp[mi][2];
     if (mi != 0)
@@ -748,6 +774,7 @@ __global__ void __launch_bounds__(kThreads, ThreadPixelBlocks<S, NB>::kMin) Loca
   pr.win = tile + ty * tw + (col - col0) + RefTileShift(R);
   float M[5][NB];
   float hyp[5][4];
+  const float mw = (float)__popc(sel & (N < 32 ? (1u << N) - 1u : 0xffffffffu));  // selected views
   int mi = -1;
   // Rounds 0..4 score five random hypotheses on the selected views; round 5
   // rescores the winner on the unselected views. One call site of the cost code.
@@ -764,21 +791,23 @@ __global__ void __launch_bounds__(kThreads, ThreadPixelBlocks<S, NB>::kMin) Loca
     // [quirk] :2916-2919 passes the inverse intrinsics where K is expected when
     // rescoring the unselected views.
     const float* Kg = (it < 5) ? p.refK : p.refiK;
-    float mconf = 0.f, mw = 0.f;
+    float mconf = 0.f;
+    bool out = false;  // the views scored so far prove the mean above conf
     for (int v = 0; v < N; ++v) {
       const bool selected = (sel >> v) & 1u;
-      if (selected != (it < 5)) continue;
+      if (selected != (it < 5) || out) continue;
       const float cost = ViewCost<R, S, 1, true>(p, poses, v, row, col, hcur[3], hcur, np, pr, Kg, 0, gmask);
       if (it < 5) {
         M[it][v] = cost;
         mconf += cost;
-        mw += 1.f;
+        out = WorseThan(mconf, conf * mw);
       } else {
         p.cost[(size_t)v * WH + pix] = cost;
       }
     }
     if (it == 5) break;
     if (mw <= 0.f) return;
+    if (out) continue;
     mconf /= mw;
     if (mconf < conf) {
       conf = mconf;
