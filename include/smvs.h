@@ -460,9 +460,10 @@ int smvs_cross_filter_synchronize(smvs_cross_filter* cf);
 void smvs_cross_filter_destroy(smvs_cross_filter* cf);
 /* Cross filters, depth-map pools (views, kept maps, job state), fusion and
  * the initial-map builders allocate from a per-device stream-ordered memory
- * pool that keeps freed memory reserved for the next call; this returns the
- * free part of it to the device (synchronises the device). gpu_index -1 =
- * current device. */
+ * pool that keeps freed memory reserved for the next call; engines allocate
+ * from a second one that keeps at most 4 GiB. This returns the free part of
+ * both to the device (synchronises the device). gpu_index -1 = current
+ * device. */
 int smvs_cross_filter_release_cache(int gpu_index);
 
 /* ---- initial depth/normal maps from the model ---------------------------- */

@@ -46,6 +46,7 @@
 
 extern "C" void smvs_internal_set_error(const char* msg);
 void smvs_internal_pose_record(const smvs_view* ref, const smvs_view* src, float* out43);
+cudaMemPool_t smvs_internal_engine_pool(int device);
 
 namespace {
 
@@ -894,6 +895,7 @@ int smvs_cross_filter_release_cache(int gpu_index) {
   if (!pool) return Fail(SMVS_ECUDA, "no memory pool on device %d", dev);
   CF_CUDA(cudaDeviceSynchronize());
   CF_CUDA(cudaMemPoolTrimTo(pool, 0));
+  if (cudaMemPool_t engines = smvs_internal_engine_pool(dev)) CF_CUDA(cudaMemPoolTrimTo(engines, 0));
   return SMVS_OK;
 }
 

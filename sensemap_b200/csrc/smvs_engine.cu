@@ -10,6 +10,8 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <map>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -22,6 +24,35 @@
 #include "smvs_kernels.h"
 
 cudaMemPool_t smvs_internal_device_pool(int device);
+
+// The memory pool of the engines of a device. An engine lives for one depth
+// map and makes some 30 allocations; cudaMalloc and cudaFree took 0.6 + 0.5 ms of
+// a 160x120 map's 2.8 ms, 8 + 7 ms at 1201x899 with 8 sources, and now and then
+// 50-240 ms (the driver maps and unmaps device memory). The pool keeps at most
+// kEngineReserve bytes between engines and returns the rest at their next
+// synchronisation; smvs_cross_filter_release_cache returns all of it.
+cudaMemPool_t smvs_internal_engine_pool(int device) {
+  constexpr uint64_t kEngineReserve = 4ull << 30;
+  static std::mutex mu;
+  static std::map<int, cudaMemPool_t> pools;
+  std::lock_guard<std::mutex> lock(mu);
+  auto it = pools.find(device);
+  if (it != pools.end()) return it->second;
+  cudaMemPoolProps props;
+  memset(&props, 0, sizeof(props));
+  props.allocType = cudaMemAllocationTypePinned;
+  props.location.type = cudaMemLocationTypeDevice;
+  props.location.id = device;
+  cudaMemPool_t pool = nullptr;
+  if (cudaMemPoolCreate(&pool, &props) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return nullptr;
+  }
+  uint64_t keep = kEngineReserve;
+  cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+  pools[device] = pool;
+  return pool;
+}
 
 namespace {
 
@@ -181,35 +212,51 @@ struct smvs_engine {
   struct Timed { int kind; cudaEvent_t start, stop; };
   std::vector<Timed> timed;
 
-  // Memory the library's per-device memory pool keeps in reserve (freed by
-  // pools, filters and fusion) is returned to the device before an allocation
-  // here reports that the device is full.
-  static bool ReleaseReserve() {
+  cudaMemPool_t mem = nullptr;  // smvs_internal_engine_pool; null: cudaMalloc
+  // Memory the library's per-device memory pools keep in reserve (freed by
+  // engines, pools, filters and fusion) is returned to the device before an
+  // allocation here reports that the device is full.
+  bool ReleaseReserve() {
     (void)cudaGetLastError();
-    int dev = 0;
-    cudaMemPool_t pool = cudaGetDevice(&dev) == cudaSuccess ? smvs_internal_device_pool(dev) : nullptr;
-    return pool && cudaDeviceSynchronize() == cudaSuccess && cudaMemPoolTrimTo(pool, 0) == cudaSuccess;
+    if (cudaDeviceSynchronize() != cudaSuccess) return false;
+    bool any = false;
+    for (cudaMemPool_t pool : {smvs_internal_device_pool(device), mem})
+      any = (pool && cudaMemPoolTrimTo(pool, 0) == cudaSuccess) || any;
+    return any;
+  }
+  cudaError_t Get(void** p, size_t bytes) {
+    return mem ? cudaMallocFromPoolAsync(p, bytes, mem, stream) : cudaMalloc(p, bytes);
   }
   int Alloc(void** p, size_t bytes) {
-    cudaError_t e = cudaMalloc(p, bytes);
-    if (e == cudaErrorMemoryAllocation && ReleaseReserve()) e = cudaMalloc(p, bytes);
-    if (e != cudaSuccess) return Fail(SMVS_ENOMEM, "cudaMalloc(%zu) failed: %s", bytes, cudaGetErrorString(e));
+    cudaError_t e = Get(p, bytes);
+    if (e == cudaErrorMemoryAllocation && ReleaseReserve()) e = Get(p, bytes);
+    if (e != cudaSuccess) return Fail(SMVS_ENOMEM, "device allocation of %zu bytes failed: %s", bytes, cudaGetErrorString(e));
     allocations.push_back(*p);
     return SMVS_OK;
   }
+  // Rows of a multiple of 512 bytes from a 512-byte boundary, as textures over
+  // pitched memory ask for (a pool block starts on a 256-byte boundary).
   int AllocPitch(void** p, size_t* pitch, size_t wbytes, int h) {
-    cudaError_t e = cudaMallocPitch(p, pitch, wbytes, (size_t)h);
-    if (e == cudaErrorMemoryAllocation && ReleaseReserve()) e = cudaMallocPitch(p, pitch, wbytes, (size_t)h);
-    if (e != cudaSuccess) return Fail(SMVS_ENOMEM, "cudaMallocPitch failed: %s", cudaGetErrorString(e));
-    allocations.push_back(*p);
-    return SMVS_OK;
+    *pitch = (wbytes + 511) & ~(size_t)511;
+    const int st = Alloc(p, *pitch * (size_t)h + 512);
+    if (st == SMVS_OK) *p = reinterpret_cast<void*>((reinterpret_cast<uintptr_t>(*p) + 511) & ~(uintptr_t)511);
+    return st;
   }
+  // Frees the device memory once no work on the device can still read it: other
+  // streams may use this engine's maps (smvs_get_device_maps) until it is closed.
   ~smvs_engine() {
-    if (stream) cudaStreamSynchronize(stream);
+    int dev = 0;
+    const bool other = cudaGetDevice(&dev) == cudaSuccess && dev != device;
+    if (other) cudaSetDevice(device);
+    if (stream) cudaDeviceSynchronize();
     for (auto& t : timed) { cudaEventDestroy(t.start); cudaEventDestroy(t.stop); }
     for (auto t : textures) cudaDestroyTextureObject(t);
-    for (auto p : allocations) cudaFree(p);
+    for (auto p : allocations) {
+      if (mem) cudaFreeAsync(p, stream); else cudaFree(p);
+    }
+    if (stream) cudaStreamSynchronize(stream);  // lets the pool return what it holds above its reserve
     if (own_stream && stream) cudaStreamDestroy(stream);
+    if (other) cudaSetDevice(dev);
   }
 };
 
@@ -429,6 +476,7 @@ int smvs_create(const smvs_options* opt, const smvs_problem* prob, void* stream,
     if (err != cudaSuccess) { delete e; return Fail(SMVS_ECUDA, "cudaStreamCreate: %s", cudaGetErrorString(err)); }
     e->own_stream = true;
   }
+  e->mem = smvs_internal_engine_pool(e->device);
   const int W = prob->ref.width, H = prob->ref.height, N = prob->num_src;
   e->W = W; e->H = H; e->N = N;
   const size_t WH = (size_t)W * H;
