@@ -638,15 +638,17 @@ int smvs_create(const smvs_options* opt, const smvs_problem* prob, void* stream,
 
 // The reference image's TMA descriptor for the job's launch shape, or
 // tma_box_w = 0 (plain loads) when the image does not qualify.
-static int UploadRefMap(smvs_engine* e, smvs::JobParams* p) {
+static int UploadRefMap(smvs_engine* e, smvs::JobParams* p, bool spread) {
   p->tma_box_w = p->tma_box_h = 0;
+  const int box_w = smvs::RefTileW(spread ? smvs::kSpreadX : p->block_x, p->R);
+  const int box_h = spread ? smvs::kSpreadRows + 2 * p->R : smvs::RefTileH(p->block_x, p->tpp, p->R);
   CUtensorMap map;
-  if (!e->use_tma || !smvs::EncodeRefMap(&map, p->ref, p->W, p->H, p->block_x, p->tpp, p->R)) return SMVS_OK;
+  if (!e->use_tma || !smvs::EncodeRefMap(&map, p->ref, p->W, p->H, box_w, box_h)) return SMVS_OK;
   // The host descriptor dies at return: copy it before returning.
   SMVS_CUDA(cudaMemcpyAsync(e->d_tmap, &map, sizeof(map), cudaMemcpyHostToDevice, e->stream));
   SMVS_CUDA(cudaStreamSynchronize(e->stream));
-  p->tma_box_w = smvs::RefTileW(p->block_x, p->R);
-  p->tma_box_h = smvs::RefTileH(p->block_x, p->tpp, p->R);
+  p->tma_box_w = box_w;
+  p->tma_box_h = box_h;
   return SMVS_OK;
 }
 
@@ -684,7 +686,9 @@ int smvs_run(smvs_engine* e) {
   if (st) return st;
   smvs::Batch b{};
   if ((st = smvs_internal_prepare_job(&p, &o))) return st;
-  if ((st = UploadRefMap(e, &p))) return st;
+  const bool spread = p.tpp == 1 && !e->persistent && p.prior_mode == 0 &&
+                      smvs::UseSpread((long long)e->W * e->H / 2, p.R, p.S, smvs::ViewBucket(p.N));
+  if ((st = UploadRefMap(e, &p, spread))) return st;
   e->tma_active = p.tma_box_w > 0;
   e->tpp_used = p.tpp;
   {
@@ -693,7 +697,7 @@ int smvs_run(smvs_engine* e) {
     int* ints = reinterpret_cast<int*>(host + sizeof(smvs::JobParams));
     memcpy(host, &p, sizeof(p));
     const int by = smvs::SweepRows(p.block_x, p.tpp);
-    const int nb = p.blocks_x * ((e->H + by - 1) / by);
+    const int nb = spread ? smvs::SpreadTiles(e->W, e->H) : p.blocks_x * ((e->H + by - 1) / by);
     const int ncb = p.conf_blocks_x * ((e->H + 7) / 8);
     ints[0] = 0;             // iteration counter
     ints[1] = 0; ints[2] = nb;   // checkerboard prefix
@@ -715,6 +719,7 @@ int smvs_run(smvs_engine* e) {
     b.status = e->d_status;
     b.tma_polls = e->tma_polls;
     b.tma_skip_copy = e->tma_skip_copy;
+    b.spread = spread;
     b.persistent = e->persistent;
     b.grid_cap = smvs::PersistentGridCap();
   }

@@ -80,6 +80,7 @@ struct Batch {
   int tma_skip_copy;            // test hook: arm the tile barrier but issue no copy (its waits run out)
   int persistent;               // tpp == 1: a persistent grid strides over the tiles (0: one block per tile)
   int grid_cap;                 // test hook: at most this many persistent blocks (0 = the resident count)
+  int spread;                   // the tiles are the spread kernels' (SpreadTiles)
 };
 
 // Checkerboard blocks: 256 threads, tpp threads per pixel, bx pixels per
@@ -92,6 +93,11 @@ __host__ __device__ inline int SweepRows(int bx, int tpp) { return 256 / (tpp * 
 __host__ __device__ inline int RefTileShift(int R) { return (4 - (R & 3)) & 3; }
 __host__ __device__ inline int RefTileW(int bx, int R) { return (2 * bx + 2 * R + RefTileShift(R) + 3) & ~3; }
 __host__ __device__ inline int RefTileH(int bx, int tpp, int R) { return SweepRows(bx, tpp) + 2 * R; }
+// The form for launches with few pixels (smvs_spread.cuh): blocks of kSpreadWarps
+// warps over tiles of kSpreadX x kSpreadRows pixels (two image columns each).
+constexpr int kSpreadWarps = 10, kSpreadX = 16, kSpreadRows = 2;
+__host__ __device__ inline int SpreadTilesX(int W) { return (W + 2 * kSpreadX - 1) / (2 * kSpreadX); }
+inline int SpreadTiles(int W, int H) { return SpreadTilesX(W) * ((H + kSpreadRows - 1) / kSpreadRows); }
 // Hypotheses per pixel of the sweep (K_NUM_SAMPS + 3, kernel_functions.h:32).
 constexpr int kSweepHyp = 11;
 // Largest dynamic shared memory a checkerboard block may request (the B200's
@@ -111,6 +117,29 @@ __host__ __device__ inline size_t LocalKernelSmem(int R, int nb, int bx, int tpp
   const size_t tile = (size_t)RefTileW(bx, R) * RefTileH(bx, tpp, R);
   return 128 + sizeof(float) * (tile + (size_t)nb * SMVS_POSE_FLOATS + P * (5 * nb));
 }
+// Same for a block of the spread form, both kernels (the sweep's need): tile,
+// poses, windows, costs, hypotheses, view weights and probabilities, costs.
+inline size_t SpreadSmemBytes(int R, int S, int nb) {
+  const size_t taps = (size_t)(2 * R / S + 1) * (2 * R / S + 1);
+  const size_t tile = (size_t)RefTileW(kSpreadX, R) * (kSpreadRows + 2 * R);
+  return 128 + sizeof(float) * (tile + (size_t)nb * SMVS_POSE_FLOATS +
+                                32 * (2 * taps + kSweepHyp * nb + kSweepHyp * 4 + 2 * nb + kSweepHyp));
+}
+// Whether a launch over `pixels` pixels of one colour (all its jobs), nb views a
+// pixel, takes the spread form (given one thread per pixel, no persistent grid
+// and no prior). Measured, thread per pixel -> spread, ms per sweep launch (pixels of a
+// colour): 2 views R=3 S=2: 5,400 0.062 -> 0.025, 21,600 0.063 -> 0.060, 38,400
+// 0.075 -> 0.094; 4 views R=5 S=2: 9,600 0.149 -> 0.062, 38,400 0.174 -> 0.159, 60,000
+// 0.215 -> 0.236; 10 views R=5 S=2: 9,600 0.347 -> 0.111, 86,400 0.719 -> 0.631, 153,600
+// 1.080 -> 1.097; 4 views R=5 S=1: 9,600 0.358 -> 0.127, 117,600 1.247 -> 1.125, 153,600
+// 1.375 -> 1.441; 10 views R=5 S=1: 9,600 0.711 -> 0.234, 240,000 4.248 -> 4.091. So the
+// line rises with the samples of a pixel's hypothesis.
+inline bool UseSpread(long long pixels, int R, int S, int nb) {
+  const long long samples = (long long)nb * (2 * R / S + 1) * (2 * R / S + 1);
+  if (samples < 100) return pixels <= 10000;
+  if (samples >= 1000) return pixels <= 200000;
+  return pixels <= 100000 && pixels <= 250 * samples;
+}
 // Same for an InitConf block (32 x 8 pixels, one thread each: the cost vector
 // and its sort order per pixel).
 __host__ __device__ inline size_t InitConfKernelSmem(int R, int nb) {
@@ -121,11 +150,11 @@ inline bool ValidSweepShape(int bx, int tpp) {
   return (bx == 8 || bx == 16 || bx == 32 || bx == 64) && (tpp == 1 || tpp == 2 || tpp == 4) && bx * tpp <= 256;
 }
 
-// Encodes the TMA descriptor of a dense W x H FP32 reference image for the
-// checkerboard tile of launch shape bx and window R. Returns false (use plain
-// loads) when the image rows are not a multiple of 16 bytes, the image is
+// Encodes the TMA descriptor of a dense W x H FP32 reference image for
+// checkerboard tiles of box_w x box_h (RefTileW, RefTileH). Returns false (use
+// plain loads) when the image rows are not a multiple of 16 bytes, the image is
 // smaller than the box, or the driver does not provide the encoder.
-bool EncodeRefMap(CUtensorMap* map, const float* ref, int W, int H, int bx, int tpp, int R);
+bool EncodeRefMap(CUtensorMap* map, const float* ref, int W, int H, int box_w, int box_h);
 
 // All launchers enqueue on `stream` and return the launch status.
 cudaError_t LaunchConvertImage(const void* in, int in_format, size_t in_stride, int w, int h, void* out,

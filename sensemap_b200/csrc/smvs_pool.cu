@@ -679,9 +679,10 @@ int Admit(smvs_pool* P, PoolJob& J) {
   }
   p.tma_box_w = p.tma_box_h = 0;
   memset(&J.map, 0, sizeof(J.map));
-  if (P->opt.ref_tile_tma && smvs::EncodeRefMap(&J.map, p.ref, W, H, p.block_x, p.tpp, p.R)) {
-    p.tma_box_w = smvs::RefTileW(p.block_x, p.R);
-    p.tma_box_h = smvs::RefTileH(p.block_x, p.tpp, p.R);
+  const int box_w = smvs::RefTileW(p.block_x, p.R), box_h = smvs::RefTileH(p.block_x, p.tpp, p.R);
+  if (P->opt.ref_tile_tma && smvs::EncodeRefMap(&J.map, p.ref, W, H, box_w, box_h)) {
+    p.tma_box_w = box_w;
+    p.tma_box_h = box_h;
   }
   J.block_bytes = JobBytes(W, H, N);
   J.block = P->arena.Reuse(J.block_bytes);  // cached blocks are already counted in bytes_used
@@ -756,6 +757,11 @@ int BuildGroups(smvs_pool* P, const std::vector<int64_t>& ids, std::vector<smvs:
     b.persistent = P->opt.sweep_persistent != 0;
     b.grid_cap = smvs::PersistentGridCap();
     const int by = smvs::SweepRows(b.block_x, b.tpp);
+    long long pixels = 0;  // of one colour, all jobs of the group
+    for (int64_t id : list) pixels += (long long)P->jobs[id].p.W * P->jobs[id].p.H / 2;
+    // (The jobs' tile descriptors are the other form's: spread tiles are staged
+    // with plain loads.)
+    b.spread = b.tpp == 1 && !b.persistent && smvs::UseSpread(pixels, b.R, b.S, b.NB);
     int tot = 0, ctot = 0;
     for (int k = 0; k < n; ++k) {
       PoolJob& J = P->jobs[list[k]];
@@ -764,7 +770,7 @@ int BuildGroups(smvs_pool* P, const std::vector<int64_t>& ids, std::vector<smvs:
       iters[base + k] = J.iter;
       prefix[pos + k] = tot;
       cprefix[pos + k] = ctot;
-      tot += J.p.blocks_x * ((J.p.H + by - 1) / by);
+      tot += b.spread ? smvs::SpreadTiles(J.p.W, J.p.H) : J.p.blocks_x * ((J.p.H + by - 1) / by);
       ctot += J.p.conf_blocks_x * ((J.p.H + 7) / 8);
     }
     prefix[pos + n] = tot;

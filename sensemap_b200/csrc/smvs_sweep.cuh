@@ -128,13 +128,13 @@ __device__ __forceinline__ bool TmaStageTile(const CUtensorMap* map, float* tile
   return false;
 }
 
-// Stage the reference tile (TMA when the job has a descriptor for this launch
+// Stage the reference tile of bx pixels a row (TMA when the job has a descriptor for this launch
 // shape, else plain loads) and the pose records. `tile` holds RefTileH rows of
 // RefTileW floats starting at (row0 - R, col0 - R - RefTileShift(R)).
 template <int R>
-__device__ __forceinline__ bool StageRefTile(const Batch& b, int job, const JobParams& p, float* tile, int row0,
-                                             int col0, int rows, float* poses, uint64_t* mbar, uint32_t& tma_uses) {
-  const int bx = b.block_x;
+__device__ __forceinline__ bool StageRefTile(const Batch& b, int job, const JobParams& p, int bx, float* tile,
+                                             int row0, int col0, int rows, float* poses, uint64_t* mbar,
+                                             uint32_t& tma_uses) {
   const int tw = RefTileW(bx, R), th = rows + 2 * R;
   const int x0 = col0 - R - RefTileShift(R), y0 = row0 - R;
   const bool tma = b.ref_maps != nullptr && p.tma_box_w == tw && p.tma_box_h == th;
@@ -466,7 +466,7 @@ __device__ __forceinline__ bool SweepTileL(const Batch& b, int colour, int bid, 
   float* tile = Align128(smem);  // a TMA destination starts on a 128-byte boundary
   float* poses = tile + tw * th;
   const int col0 = (blk % p.blocks_x) * 2 * kBX, row0 = (blk / p.blocks_x) * kBY;
-  if (!StageRefTile<R>(b, job, p, tile, row0, col0, kBY, poses, mbar, tma_uses)) return false;  // block-uniform
+  if (!StageRefTile<R>(b, job, p, b.block_x, tile, row0, col0, kBY, poses, mbar, tma_uses)) return false;  // block-uniform
   __syncthreads();
   const int tx = threadIdx.x % kBX, ty = threadIdx.x / kBX;
   const int row = row0 + ty;
@@ -734,7 +734,7 @@ __global__ void __launch_bounds__(kThreads, ThreadPixelBlocks<S, NB>::kMin) Loca
   float* poses = tile + tw * th;
   const int col0 = (blk % p.blocks_x) * 2 * kBX, row0 = (blk / p.blocks_x) * kBY;
   uint32_t tma_uses = 0;
-  if (!StageRefTile<R>(b, job, p, tile, row0, col0, kBY, poses, &mbar, tma_uses)) return;  // block-uniform
+  if (!StageRefTile<R>(b, job, p, b.block_x, tile, row0, col0, kBY, poses, &mbar, tma_uses)) return;  // block-uniform
   __syncthreads();
   const int tx = threadIdx.x % kBX, ty = threadIdx.x / kBX;
   const int row = row0 + ty;
@@ -858,7 +858,7 @@ __global__ void __launch_bounds__(kThreads, SweepOccupancy<G>::kBlocks) SweepKer
   sm.PR = sm.VW + nb * P;
   const int col0 = (blk % p.blocks_x) * 2 * bx, row0 = (blk / p.blocks_x) * rows;
   uint32_t tma_uses = 0;
-  if (!StageRefTile<R>(b, job, p, tile, row0, col0, rows, poses, &mbar, tma_uses)) return;  // block-uniform
+  if (!StageRefTile<R>(b, job, p, b.block_x, tile, row0, col0, rows, poses, &mbar, tma_uses)) return;  // block-uniform
   __syncthreads();
   const int g = threadIdx.x / G, lane = threadIdx.x % G;
   const int row = row0 + g / bx;
@@ -1095,7 +1095,7 @@ __global__ void __launch_bounds__(kThreads, SweepOccupancy<G>::kBlocks) LocalOpt
   float* Ms = poses + nb * SMVS_POSE_FLOATS;  // [5][nb][P]
   const int col0 = (blk % p.blocks_x) * 2 * bx, row0 = (blk / p.blocks_x) * rows;
   uint32_t tma_uses = 0;
-  if (!StageRefTile<R>(b, job, p, tile, row0, col0, rows, poses, &mbar, tma_uses)) return;  // block-uniform
+  if (!StageRefTile<R>(b, job, p, b.block_x, tile, row0, col0, rows, poses, &mbar, tma_uses)) return;  // block-uniform
   __syncthreads();
   const int g = threadIdx.x / G, lane = threadIdx.x % G;
   const int row = row0 + g / bx;
@@ -1188,6 +1188,16 @@ __global__ void __launch_bounds__(kThreads, SweepOccupancy<G>::kBlocks) LocalOpt
 
 static_assert(kSweepHyp == kMaxHyp, "hypotheses per pixel");
 
+}  // namespace
+}  // namespace detail
+}  // namespace smvs
+
+#include "smvs_spread.cuh"
+
+namespace smvs {
+namespace detail {
+namespace {
+
 template <int R, int S, int G>
 cudaError_t LaunchSweepT(const Batch& b, int colour, bool local, cudaStream_t stream) {
   if (b.total_blocks <= 0) return cudaSuccess;
@@ -1233,6 +1243,7 @@ cudaError_t LaunchSweepL(const Batch& b, int colour, bool local, cudaStream_t st
 
 template <int R, int S>
 cudaError_t LaunchSweepG(const Batch& b, int colour, bool local, cudaStream_t stream) {
+  if (b.spread) return LaunchSpread<R, S>(b, colour, local, stream);
   if (b.tpp == 1) {
     if (b.NB <= 8) return LaunchSweepL<R, S, 8>(b, colour, local, stream);
     if (b.NB <= 12) return LaunchSweepL<R, S, 12>(b, colour, local, stream);
@@ -1271,6 +1282,8 @@ template <int R, int S>
 cudaError_t ConfigureWindow() {
   cudaError_t e = cudaSuccess;
   if (e == cudaSuccess) e = AllowLargeSmem(InitConfKernel<R, S>);
+  if (e == cudaSuccess) e = AllowLargeSmem(SweepKernelSpread<R, S>);
+  if (e == cudaSuccess) e = AllowLargeSmem(LocalOptKernelSpread<R, S>);
   if (e == cudaSuccess) e = AllowLargeSmem(SweepKernel<R, S, 2>);
   if (e == cudaSuccess) e = AllowLargeSmem(SweepKernel<R, S, 4>);
   if (e == cudaSuccess) e = AllowLargeSmem(LocalOptKernel<R, S, 2>);
