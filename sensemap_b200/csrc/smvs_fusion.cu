@@ -135,7 +135,7 @@ struct FImage {
 };
 
 // Record pool of one image. A record (u32 words): cnt, nE, gid[cnt], derr[cnt],
-// pred[cnt], eoff[cnt + 1], vid[cnt] (u16), edges[nE bound] (u16).
+// eoff[cnt + 1], vid[cnt] (u16), edges[nE bound] (u16).
 struct FRecs {
   uint32_t* pool;
   unsigned long long pool_words;
@@ -147,7 +147,7 @@ struct FRecs {
 };
 
 __host__ __device__ inline uint32_t RecWords(uint32_t cnt, uint32_t ebound) {
-  return 2u + 3u * cnt + (cnt + 1u) + (cnt + 1u) / 2u + (ebound + 1u) / 2u;
+  return 2u + 2u * cnt + (cnt + 1u) + (cnt + 1u) / 2u + (ebound + 1u) / 2u;
 }
 
 // Bytes of one replay warp's scratch region: stack (u32) | vals (f32) | ids (u32)
@@ -363,14 +363,12 @@ __device__ bool WriteRecord(const FMaps& m, const FRecs& r, uint32_t seed, const
   uint32_t* rec = r.pool + off;
   uint32_t* rg = rec + 2;
   float* rd = reinterpret_cast<float*>(rg + cnt);
-  int32_t* rp = reinterpret_cast<int32_t*>(rd + cnt);
-  uint32_t* eoff = reinterpret_cast<uint32_t*>(rp + cnt);
+  uint32_t* eoff = reinterpret_cast<uint32_t*>(rd + cnt);
   uint16_t* rv = reinterpret_cast<uint16_t*>(eoff + cnt + 1);
   uint16_t* edges = rv + 2 * ((cnt + 1) / 2);
   for (int i = 0; i < cnt; ++i) {
     rg[i] = gid[i];
     rd[i] = derr[i];
-    rp[i] = -1;
     rv[i] = vid[i];
   }
   uint32_t e = 0;
@@ -622,14 +620,12 @@ __global__ void __launch_bounds__(32 * kClosureWarps) ClosureKernel(FMaps m, FCo
     uint32_t* rec = r.pool + off;
     uint32_t* rg = rec + 2;
     float* rd = reinterpret_cast<float*>(rg + cnt);
-    int32_t* rpd = reinterpret_cast<int32_t*>(rd + cnt);
-    uint32_t* reo = reinterpret_cast<uint32_t*>(rpd + cnt);
+    uint32_t* reo = reinterpret_cast<uint32_t*>(rd + cnt);
     uint16_t* rv = reinterpret_cast<uint16_t*>(reo + cnt + 1);
     uint16_t* redg = rv + 2 * ((cnt + 1) / 2);
     for (int k = lane; k < cnt; k += 32) {
       rg[k] = sh.gid[k];
       rd[k] = derr[k];
-      rpd[k] = -1;
       rv[k] = sh.vid[k];
     }
     for (int k = lane; k <= cnt; k += 32) reo[k] = eoff[k];
@@ -674,7 +670,6 @@ struct RecView {
   uint32_t cnt, ne;
   const uint32_t* gid;
   const float* derr;
-  int32_t* pred;
   const uint32_t* eoff;
   const uint16_t* vid;
   const uint16_t* edges;
@@ -687,8 +682,7 @@ __device__ __forceinline__ RecView OpenRecord(uint32_t* pool, uint32_t off) {
   v.ne = rec[1];
   v.gid = rec + 2;
   v.derr = reinterpret_cast<const float*>(v.gid + v.cnt);
-  v.pred = reinterpret_cast<int32_t*>(rec + 2 + 2 * v.cnt);
-  v.eoff = rec + 2 + 3 * v.cnt;
+  v.eoff = rec + 2 + 2 * v.cnt;
   v.vid = reinterpret_cast<const uint16_t*>(v.eoff + v.cnt + 1);
   v.edges = v.vid + 2 * ((v.cnt + 1) / 2);
   return v;
@@ -722,61 +716,95 @@ __global__ void __launch_bounds__(256) ClaimFillKernel(FRecs r, uint32_t nseeds,
   }
 }
 
-// Predecessor of each (seed, pixel) and the shear K of the ticket order:
-// key(p) < key(s) for every predecessor p of s needs K (i_s - i_p) > j_p - j_s.
-// The record's predecessors are written once each at the front of pred[] (the
-// replay only waits for them), the rest -1; the first 64 distinct ones are
-// recognised as repeats, any beyond that may repeat.
-constexpr int kPredSeen = 64;
+// The predecessors of a seed are the earlier seeds that claim one of its pixels,
+// each once (the replay waits for all of them). They are listed as the pixels of
+// those seeds, whose masks the replay polls: a seed is settled once its own
+// pixel is fused. Also the shear K of the ticket order: key(p) < key(s) for every
+// predecessor p of s needs K (i_s - i_p) > j_p - j_s.
+struct FPreds {
+  uint32_t* off;   // per seed: first entry in list
+  uint32_t* cnt;   // per seed: entries, or kWalk: walk the claims of the record's pixels
+  uint32_t* list;  // seed pixels
+  unsigned long long* used;
+  unsigned long long cap;
+  const uint32_t* claim_off;
+  const uint32_t* claim_list;
+};
+constexpr uint32_t kWalk = 0xffffffffu;
+constexpr int kPredSlots = 512;  // hash slots of a seed's distinct predecessors
+constexpr int kPredMost = 384;   // with more of them the replay walks the claims
 
-__global__ void __launch_bounds__(256) PredKernel(FRecs r, uint32_t nseeds, int Cs, const uint32_t* claim_off,
-                                                  const uint32_t* claim_list, int* shear) {
-  __shared__ int32_t seen_all[8][kPredSeen];
+__global__ void __launch_bounds__(256) PredKernel(FMaps m, FImage im, FRecs r, FPreds pr, int* shear) {
+  __shared__ uint32_t keys_all[8][kPredSlots];
+  __shared__ uint32_t count_all[8];
   const uint32_t s = (uint32_t)(((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
   const uint32_t lane = threadIdx.x & 31;
-  int32_t* seen = seen_all[threadIdx.x >> 5];
-  if (s >= nseeds) return;
+  uint32_t* keys = keys_all[threadIdx.x >> 5];
+  volatile uint32_t* count = count_all + (threadIdx.x >> 5);
+  if (s >= im.nseeds) return;
   const uint32_t off = r.rec_off[s];
   if (off >= kRetry) return;
-  RecView v = OpenRecord(r.pool, off);
-  const int is = (int)(s / (uint32_t)Cs), js = (int)(s - (uint32_t)is * (uint32_t)Cs);
-  const unsigned lt = (1u << lane) - 1u;
-  int need = 1;
-  uint32_t nu = 0;
-  for (uint32_t k0 = 0; k0 < v.cnt; k0 += 32) {
-    const uint32_t k = k0 + lane;
-    int32_t best = -1;
-    if (k < v.cnt) {
-      // The latest earlier claimant of this pixel (the list is in no order).
-      const uint32_t g = v.gid[k];
-      for (uint32_t q = claim_off[g], end = claim_off[g + 1]; q < end; ++q) {
-        const uint32_t cl = claim_list[q];
-        if (cl < s && (int32_t)cl > best) best = (int32_t)cl;
+  const RecView v = OpenRecord(r.pool, off);
+  for (int i = lane; i < kPredSlots; i += 32) keys[i] = kNoKey;
+  if (lane == 0) *count = 0;
+  __syncwarp();
+  for (uint32_t k = lane; k < v.cnt; k += 32) {
+    const uint32_t g = v.gid[k];
+    for (uint32_t q = pr.claim_off[g], end = pr.claim_off[g + 1]; q < end; ++q) {
+      const uint32_t cl = pr.claim_list[q];
+      if (cl >= s || *count > (uint32_t)kPredMost) continue;  // the table never fills up
+      uint32_t h = (cl * 0x9E3779B1u) >> 23;  // 512 slots
+      const volatile uint32_t* vk = keys;
+      for (;;) {
+        uint32_t key = vk[h];
+        if (key == kNoKey) key = atomicCAS(keys + h, kNoKey, cl);
+        if (key == kNoKey) { atomicAdd(count_all + (threadIdx.x >> 5), 1u); break; }
+        if (key == cl) break;
+        h = (h + 1) & (uint32_t)(kPredSlots - 1);
       }
     }
-    bool fresh = best >= 0;
-    const uint32_t known = nu < (uint32_t)kPredSeen ? nu : (uint32_t)kPredSeen;
-    for (uint32_t t = 0; fresh && t < known; ++t)
-      if (seen[t] == best) fresh = false;
-    const unsigned same = __match_any_sync(0xffffffffu, best);
-    fresh = fresh && (same & lt) == 0;  // the first lane holding this value
-    const unsigned nw = __ballot_sync(0xffffffffu, fresh);
-    if (fresh) {
-      const uint32_t pos = nu + (uint32_t)__popc(nw & lt);
-      v.pred[pos] = best;  // pos <= k: this kernel reads no pred[] entry
-      if (pos < (uint32_t)kPredSeen) seen[pos] = best;
-      const uint32_t p = (uint32_t)best;
-      const int ip = (int)(p / (uint32_t)Cs), jp = (int)(p - (uint32_t)ip * (uint32_t)Cs);
-      if (ip < is) {
-        const int num = jp - js, den = is - ip;
-        const int fl = num >= 0 ? num / den : -((-num + den - 1) / den);
-        need = max(need, fl + 1);
-      }
-    }
-    nu += (uint32_t)__popc(nw);
-    __syncwarp();
   }
-  for (uint32_t k = nu + lane; k < v.cnt; k += 32) v.pred[k] = -1;
+  __syncwarp();
+  const uint32_t n = *count;
+  unsigned long long at = 0;
+  if (lane == 0 && n > 0 && n <= (uint32_t)kPredMost) at = atomicAdd(pr.used, (unsigned long long)n);
+  at = __shfl_sync(0xffffffffu, at, 0);
+  const bool walk = n > (uint32_t)kPredMost || at + n > pr.cap;
+  if (lane == 0) {
+    pr.off[s] = (uint32_t)at;
+    pr.cnt[s] = walk ? kWalk : n;
+  }
+  // The list, and what the distinct predecessors need of the shear (with more
+  // than kPredMost, of every claim).
+  const int Cs = im.Cs;
+  const int is = (int)(s / (uint32_t)Cs), js = (int)(s - (uint32_t)is * (uint32_t)Cs);
+  int need = 1;
+  auto shear_of = [&](uint32_t p) {
+    const int ip = (int)(p / (uint32_t)Cs), jp = (int)(p - (uint32_t)ip * (uint32_t)Cs);
+    if (ip < is) {
+      const int num = jp - js, den = is - ip;
+      const int fl = num >= 0 ? num / den : -((-num + den - 1) / den);
+      need = max(need, fl + 1);
+    }
+  };
+  if (n > (uint32_t)kPredMost) {
+    for (uint32_t k = lane; k < v.cnt; k += 32) {
+      const uint32_t g = v.gid[k];
+      for (uint32_t q = pr.claim_off[g], end = pr.claim_off[g + 1]; q < end; ++q)
+        if (pr.claim_list[q] < s) shear_of(pr.claim_list[q]);
+    }
+  } else if (n > 0) {
+    uint32_t pos = 0;
+    for (int i0 = 0; i0 < kPredSlots; i0 += 32) {
+      const uint32_t p = keys[i0 + lane];
+      const unsigned has = __ballot_sync(0xffffffffu, p != kNoKey);
+      if (p != kNoKey) {
+        shear_of(p);
+        if (!walk) pr.list[at + pos + (uint32_t)__popc(has & ((1u << lane) - 1u))] = SeedPixel(m, im, p);
+      }
+      pos += (uint32_t)__popc(has);
+    }
+  }
   for (int o = 16; o > 0; o >>= 1) need = max(need, __shfl_xor_sync(0xffffffffu, need, o));
   if (lane == 0 && need > 1) atomicMax(shear, min(need, Cs));
 }
@@ -809,7 +837,8 @@ __global__ void SeqKernel(uint32_t nseeds, int Cs, const int* shear, const uint3
 struct FReplay {
   const uint32_t* seq;
   uint32_t nseeds;
-  uint32_t* done;
+  FImage im;
+  FPreds preds;
   unsigned int* ticket;
   smvs_fused_point* slot_pts;
   uint32_t* slot_has;
@@ -822,7 +851,7 @@ struct FReplay {
   uint32_t scratch_stack;     // stack capacity of a scratch region
   int shared_cnt;             // records up to this many pixels ...
   int shared_stack;           // ... and stack entries replay in shared memory
-  uint32_t* level;            // with profiling: dependency depth of each seed (else null)
+  uint32_t* level;            // with profiling: dependency depth by seed pixel of the image (else null)
   uint32_t* chain;            // with profiling: the image's longest dependency chain
   unsigned long long* times;  // with profiling: summed ns [waiting, after the wait until release], seeds
   unsigned long long wait_limit_ns;  // bound of a predecessor wait
@@ -844,13 +873,13 @@ struct WarpShared {
   int nacc;
 };
 
-__device__ __forceinline__ uint32_t LoadAcquire(const uint32_t* p) {
+__device__ __forceinline__ uint32_t LoadMask(const uint8_t* p) {
   uint32_t v;
-  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  asm volatile("ld.relaxed.gpu.global.u8 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
   return v;
 }
-__device__ __forceinline__ void StoreRelease(uint32_t* p, uint32_t v) {
-  asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+__device__ __forceinline__ void StoreMask(uint8_t* p) {
+  asm volatile("st.relaxed.gpu.global.u8 [%0], %1;" ::"l"(p), "r"(1u) : "memory");
 }
 __device__ __forceinline__ unsigned long long GlobalTimer() {
   unsigned long long t;
@@ -878,20 +907,31 @@ __device__ float WarpMedian(const float* vals, int n, float* med, int lane) {
   return r;
 }
 
-// Waits until *flag is set: a short spin, then a growing back-off (fewer loads
-// for L2 to serve while most warps wait), bounded in time (status bit on
-// timeout).
-__device__ __forceinline__ void WaitDone(const uint32_t* flag, uint32_t* stats, unsigned long long limit_ns) {
+// Waits until the masks of the seed pixels that the lanes hold (`pending` lanes)
+// are set, or the seed's own pixel is (true: another seed fused it, nothing is
+// left to do). A short spin, then a back-off; bounded in time (status bit on
+// timeout). Called by the whole warp.
+__device__ __forceinline__ bool WaitSettled(const uint8_t* mask, uint32_t own, uint32_t pixel, bool pending,
+                                            uint32_t* stats, unsigned long long limit_ns) {
+  const int lane = threadIdx.x & 31;
   unsigned long long t0 = 0;
-  unsigned ns = 0;
-  for (uint32_t it = 0; LoadAcquire(flag) == 0u; ++it) {
-    if (it < 1024) continue;
-    if (ns == 0) t0 = GlobalTimer();
-    ns = ns < 256 ? ns + 32 : 256;
-    __nanosleep(ns);
-    if (GlobalTimer() - t0 > limit_ns) {
-      atomicOr(&stats[2], kStTimeout);
-      return;
+  for (uint32_t it = 0;; ++it) {
+    bool fused = false;
+    if (pending && LoadMask(mask + pixel)) pending = false;
+    if (lane == 31) fused = LoadMask(mask + own) != 0u;
+    const unsigned open = __ballot_sync(0xffffffffu, pending);
+    if (__any_sync(0xffffffffu, fused)) return true;
+    if (!open) return false;
+    if (it < 16) continue;
+    __nanosleep(it < 64 ? 32 : 128);
+    if ((it & 63u) != 16u) continue;
+    const unsigned long long t = __shfl_sync(0xffffffffu, GlobalTimer(), 0);
+    if (t0 == 0) t0 = t;
+    // One wait that gave up ends the others too.
+    const uint32_t status = *(volatile const uint32_t*)(stats + 2);
+    if (t - t0 > limit_ns || __any_sync(0xffffffffu, (status & kStTimeout) != 0u)) {
+      if (lane == 0) atomicOr(&stats[2], kStTimeout);
+      return false;
     }
   }
 }
@@ -948,6 +988,8 @@ __global__ void __launch_bounds__(32 * kReplayWarps) ReplayKernel(FMaps m, FCons
     const uint32_t s = rp.seq[t];
     const uint32_t off = r.rec_off[s];
     if (off >= kRetry) continue;  // no record: nothing to fuse, nobody waits for it
+    const uint32_t own = SeedPixel(m, rp.im, s);
+    if (__any_sync(0xffffffffu, LoadMask(m.mask + own) != 0u)) continue;  // fused by an earlier seed
     const RecView v = OpenRecord(r.pool, off);
     const int cnt = (int)v.cnt;
     // Storage: the per-pixel arrays in shared memory when the record has at
@@ -960,7 +1002,7 @@ __global__ void __launch_bounds__(32 * kReplayWarps) ReplayKernel(FMaps m, FCons
         ((!node_sh || !stack_sh) && !rp.scratch)) {
       if (lane == 0) {
         atomicOr(&r.stats[2], kStBad);
-        StoreRelease(&rp.done[s], 1u);
+        StoreMask(m.mask + own);
       }
       continue;
     }
@@ -997,27 +1039,33 @@ __global__ void __launch_bounds__(32 * kReplayWarps) ReplayKernel(FMaps m, FCons
     unsigned long long tw0 = 0;
     if (rp.times) tw0 = GlobalTimer();
     // Wait for the predecessors (every earlier seed that may touch these
-    // pixels; the distinct ones come first in pred[]). Lane 0 waits for the
-    // latest of them, usually the last to finish; then every lane checks its
-    // own entries.
-    {
-      int32_t latest = -1;
-      for (int k = lane; k < cnt; k += 32) {
-        const int32_t p = v.pred[k];
-        if (p < 0) break;
-        latest = max(latest, p);
+    // pixels) until each is settled: it has run, or an earlier seed fused its
+    // pixel and it never will. A seed marks its own pixel last, so all its marks
+    // are visible then; a seed fused by another leaves none. The wait ends at
+    // once when another seed has fused this one's pixel.
+    bool fused = false;
+    const uint32_t npred = rp.preds.cnt[s];
+    if (npred != kWalk) {
+      const uint32_t* list = rp.preds.list + rp.preds.off[s];
+      for (uint32_t k0 = 0; k0 < npred && !fused; k0 += 32) {
+        const bool some = k0 + lane < npred;
+        fused = WaitSettled(m.mask, own, some ? list[k0 + lane] : own, some, r.stats, rp.wait_limit_ns);
       }
-      for (int o = 16; o > 0; o >>= 1) latest = max(latest, __shfl_xor_sync(0xffffffffu, latest, o));
-      if (lane == 0 && latest >= 0) WaitDone(rp.done + latest, r.stats, rp.wait_limit_ns);
-      __syncwarp();
-      for (int k = lane; k < cnt; k += 32) {
-        const int32_t p = v.pred[k];
-        if (p < 0) break;
-        WaitDone(rp.done + p, r.stats, rp.wait_limit_ns);
+    } else {
+      for (int k = 0; k < cnt && !fused; ++k) {
+        const uint32_t g = v.gid[k];
+        const uint32_t c1 = rp.preds.claim_off[g + 1];
+        for (uint32_t q0 = rp.preds.claim_off[g]; q0 < c1 && !fused; q0 += 32) {
+          const uint32_t cl = q0 + lane < c1 ? rp.preds.claim_list[q0 + lane] : s;
+          fused = WaitSettled(m.mask, own, cl < s ? SeedPixel(m, rp.im, cl) : own, cl < s, r.stats,
+                              rp.wait_limit_ns);
+        }
       }
     }
-    // The acquires above order the predecessors' mask writes before these
-    // reads for the whole warp (the barrier orders the lanes).
+    if (fused) continue;
+    // Orders the predecessors' marks, seen above, before these reads for the
+    // whole warp (the barrier orders the lanes).
+    __threadfence();
     __syncwarp();
     unsigned long long tw1 = 0;
     if (rp.times) tw1 = GlobalTimer();
@@ -1037,14 +1085,12 @@ __global__ void __launch_bounds__(32 * kReplayWarps) ReplayKernel(FMaps m, FCons
     }
     if (rp.level) {  // profiling: the longest chain of waits ending at this seed
       uint32_t lv = 0;
-      for (int k = lane; k < cnt; k += 32) {
-        const int32_t p = v.pred[k];
-        if (p < 0) break;
-        lv = max(lv, *(volatile const uint32_t*)(rp.level + p));
-      }
+      const uint32_t base_px = m.views[rp.im.view].base;
+      for (uint32_t k = lane; npred != kWalk && k < npred; k += 32)
+        lv = max(lv, *(volatile const uint32_t*)(rp.level + (rp.preds.list[rp.preds.off[s] + k] - base_px)));
       for (int o = 16; o > 0; o >>= 1) lv = max(lv, __shfl_xor_sync(0xffffffffu, lv, o));
       if (lane == 0) {
-        rp.level[s] = lv + 1;
+        rp.level[own - base_px] = lv + 1;
         atomicMax(rp.chain, lv + 1);
       }
     }
@@ -1152,11 +1198,15 @@ __global__ void __launch_bounds__(32 * kReplayWarps) ReplayKernel(FMaps m, FCons
     const int n = sh.nacc;
     unsigned long long tw_b = 0;
     if (rp.times) tw_b = GlobalTimer();
-    for (int i = lane; i < n; i += 32) *(volatile uint8_t*)(m.mask + rgid[acc[i]]) = 1;
-    // Release the successors: the barrier orders every lane's mask writes
-    // before lane 0's release store.
+    for (int i = lane; i < n; i += 32)
+      if (acc[i] != 0) *(volatile uint8_t*)(m.mask + rgid[acc[i]]) = 1;
+    // The seed's own pixel last, which releases the successors: the barrier and
+    // the fence order every lane's marks before it.
     __syncwarp();
-    if (lane == 0 && rp.withhold != -2 && (long long)s != rp.withhold) StoreRelease(&rp.done[s], 1u);
+    if (lane == 0 && rp.withhold != -2 && (long long)s != rp.withhold) {
+      __threadfence();
+      StoreMask(m.mask + own);
+    }
     if (rp.times && lane == 0) {
       const unsigned long long tw2 = GlobalTimer();
       atomicAdd(rp.times, tw1 - tw0);
@@ -1418,7 +1468,9 @@ struct smvs_fusion {
   size_t claim_list_cap = 0;
   uint32_t* d_pool = nullptr;
   size_t pool_words = 0;
-  uint32_t *d_rec_off = nullptr, *d_over_list = nullptr, *d_seq = nullptr, *d_done = nullptr;
+  uint32_t *d_rec_off = nullptr, *d_over_list = nullptr, *d_seq = nullptr;
+  uint32_t *d_pred_off = nullptr, *d_pred_cnt = nullptr, *d_pred_list = nullptr;
+  unsigned long long* d_pred_used = nullptr;
   uint32_t *d_keycnt = nullptr, *d_keyoff = nullptr;
   size_t key_cap = 0;
   smvs_fused_point* d_slot_pts = nullptr;
@@ -1523,7 +1575,8 @@ void FreeAll(smvs_fusion* f) {
     Free(f, f->d_NX); Free(f, f->d_NY); Free(f, f->d_NZ); Free(f, f->d_G);
     Free(f, f->d_rgb); Free(f, f->d_mask);
     Free(f, f->d_claim_cnt); Free(f, f->d_claim_off); Free(f, f->d_claim_list);
-    Free(f, f->d_pool); Free(f, f->d_rec_off); Free(f, f->d_over_list); Free(f, f->d_seq); Free(f, f->d_done);
+    Free(f, f->d_pool); Free(f, f->d_rec_off); Free(f, f->d_over_list); Free(f, f->d_seq);
+    Free(f, f->d_pred_off); Free(f, f->d_pred_cnt); Free(f, f->d_pred_list); Free(f, f->d_pred_used);
     Free(f, f->d_keycnt); Free(f, f->d_keyoff);
     Free(f, f->d_slot_pts); Free(f, f->d_slot_has); Free(f, f->d_slot_nvis); Free(f, f->d_slot_visoff);
     Free(f, f->d_pt_idx); Free(f, f->d_vis_idx); Free(f, f->d_vis_pool);
@@ -1641,16 +1694,29 @@ FRecs Recs(const smvs_fusion* f) {
   return r;
 }
 
+FPreds Preds(const smvs_fusion* f) {
+  FPreds p;
+  p.off = f->d_pred_off;
+  p.cnt = f->d_pred_cnt;
+  p.list = f->d_pred_list;
+  p.used = f->d_pred_used;
+  p.cap = std::min<unsigned long long>(f->claim_list_cap, 0xffffffffull);
+  p.claim_off = f->d_claim_off;
+  p.claim_list = f->d_claim_list;
+  return p;
+}
+
 // Per-seed arrays for an image of n seeds.
 int EnsureSeeds(smvs_fusion* f, uint64_t n, uint64_t nkeys) {
   int st = SMVS_OK;
   if (n > f->seed_cap) {
-    Free(f, f->d_rec_off); Free(f, f->d_over_list); Free(f, f->d_seq); Free(f, f->d_done);
+    Free(f, f->d_rec_off); Free(f, f->d_over_list); Free(f, f->d_seq);
+    Free(f, f->d_pred_off); Free(f, f->d_pred_cnt);
     Free(f, f->d_slot_pts); Free(f, f->d_slot_has); Free(f, f->d_slot_nvis); Free(f, f->d_slot_visoff);
     Free(f, f->d_pt_idx); Free(f, f->d_vis_idx);
     f->seed_cap = n;
     if ((st = Alloc(f, &f->d_rec_off, n)) || (st = Alloc(f, &f->d_over_list, n)) || (st = Alloc(f, &f->d_seq, n)) ||
-        (st = Alloc(f, &f->d_done, n)) || (st = Alloc(f, &f->d_slot_pts, n)) || (st = Alloc(f, &f->d_slot_has, n)) ||
+        (st = Alloc(f, &f->d_pred_off, n)) || (st = Alloc(f, &f->d_pred_cnt, n)) || (st = Alloc(f, &f->d_slot_pts, n)) || (st = Alloc(f, &f->d_slot_has, n)) ||
         (st = Alloc(f, &f->d_slot_nvis, n)) || (st = Alloc(f, &f->d_slot_visoff, n)) ||
         (st = Alloc(f, &f->d_pt_idx, n + 1)) || (st = Alloc(f, &f->d_vis_idx, n + 1))) {
       f->seed_cap = 0;
@@ -1773,19 +1839,23 @@ int FuseImage(smvs_fusion* f, int image) {
   // 2. Claims and predecessors.
   {
     ProfScope ps(f, SMVS_FUSION_KERNEL_ORDER);
-    const uint64_t claims = used / 4 + 1;  // a record of cnt pixels takes more than 4 cnt words
+    const uint64_t claims = used / 3 + 1;  // a record of cnt pixels takes more than 3 cnt words
     if (claims > f->claim_list_cap) {
       Free(f, f->d_claim_list);
+      Free(f, f->d_pred_list);
       f->claim_list_cap = (size_t)claims + 1024;
-      if ((st = Alloc(f, &f->d_claim_list, f->claim_list_cap))) { f->claim_list_cap = 0; return st; }
+      if ((st = Alloc(f, &f->d_claim_list, f->claim_list_cap)) || (st = Alloc(f, &f->d_pred_list, f->claim_list_cap))) {
+        f->claim_list_cap = 0;
+        return st;
+      }
     }
     ClaimCountKernel<<<Blocks(32 * nseeds, 256), 256, 0, f->stream>>>(Recs(f), (uint32_t)nseeds, f->d_claim_cnt);
     ++f->launches;
     if ((st = Scan(f, f->d_claim_cnt, f->total, f->d_claim_off))) return st;
     ClaimFillKernel<<<Blocks(32 * nseeds, 256), 256, 0, f->stream>>>(Recs(f), (uint32_t)nseeds, f->d_claim_cnt,
                                                                  f->d_claim_off, f->d_claim_list);
-    PredKernel<<<Blocks(32 * nseeds, 256), 256, 0, f->stream>>>(Recs(f), (uint32_t)nseeds, Cs, f->d_claim_off,
-                                                           f->d_claim_list, f->d_shear);
+    FU_CUDA(cudaMemsetAsync(f->d_pred_used, 0, sizeof(unsigned long long), f->stream));
+    PredKernel<<<Blocks(32 * nseeds, 256), 256, 0, f->stream>>>(m, im, Recs(f), Preds(f), f->d_shear);
     // 3. Ticket order.
     KeyCountKernel<<<Blocks(nkeys, 256), 256, 0, f->stream>>>((uint32_t)nkeys, Rs, Cs, f->d_shear, f->d_keycnt);
     f->launches += 3;
@@ -1807,14 +1877,14 @@ int FuseImage(smvs_fusion* f, int image) {
     f->replay_scratch_cnt = cap_cnt;
     f->replay_scratch_stack = cap_stack;
   }
-  FU_CUDA(cudaMemsetAsync(f->d_done, 0, nseeds * sizeof(uint32_t), f->stream));
   FU_CUDA(cudaMemsetAsync(f->d_slot_has, 0, nseeds * sizeof(uint32_t), f->stream));
   FU_CUDA(cudaMemsetAsync(f->d_slot_nvis, 0, nseeds * sizeof(uint32_t), f->stream));
   {
     FReplay rp;
     rp.seq = f->d_seq;
     rp.nseeds = (uint32_t)nseeds;
-    rp.done = f->d_done;
+    rp.im = im;
+    rp.preds = Preds(f);
     rp.ticket = f->d_ticket;
     rp.slot_pts = f->d_slot_pts;
     rp.slot_has = f->d_slot_has;
@@ -1833,11 +1903,13 @@ int FuseImage(smvs_fusion* f, int image) {
     rp.wait_limit_ns = t_wait_limit_ns ? t_wait_limit_ns : kWaitLimitNs;
     rp.withhold = t_withhold;
     if (f->profiling) {
-      if (nseeds > f->level_cap) {
+      const size_t plane = (size_t)W * (size_t)H;
+      if (plane > f->level_cap) {
         Free(f, f->d_level);
-        f->level_cap = nseeds;
-        if ((st = Alloc(f, &f->d_level, nseeds))) { f->level_cap = 0; return st; }
+        f->level_cap = plane;
+        if ((st = Alloc(f, &f->d_level, plane))) { f->level_cap = 0; return st; }
       }
+      FU_CUDA(cudaMemsetAsync(f->d_level, 0, plane * sizeof(uint32_t), f->stream));
       if (!f->d_chain && (st = Alloc(f, &f->d_chain, 2 * (size_t)f->num_views))) return st;
       const int k = (int)f->order.size();
       FU_CUDA(cudaMemsetAsync(f->d_chain + k, 0, sizeof(uint32_t), f->stream));
@@ -2161,6 +2233,7 @@ int smvs_fusion_create(const smvs_fusion_options* opt, const smvs_fusion_view* v
       (st = Alloc(f, &f->d_out_pts, T / 2 + 1)) || (st = Alloc(f, &f->d_out_visoff, T / 2 + 2)) ||
       (st = Alloc(f, &f->d_out_vis, T)) || (st = Alloc(f, &f->d_shear, 1)) || (st = Alloc(f, &f->d_ticket, 1)) ||
       (st = Alloc(f, &f->d_n_over, 1)) || (st = Alloc(f, &f->d_stats, 3)) || (st = Alloc(f, &f->d_used, 1)) ||
+      (st = Alloc(f, &f->d_pred_used, 1)) ||
       (st = Alloc(f, &f->d_vis_cursor, 1)) || (st = Alloc(f, &f->d_totals, 2)))
     return fail(st);
   if (opt->with_normal &&
