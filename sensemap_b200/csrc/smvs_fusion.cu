@@ -15,17 +15,16 @@
 //      them in the reference's push order (the seed's record); records over
 //      the shared capacity take a thread-per-seed overflow pass;
 //   2. claims: for every pixel the seeds whose records hold it; each seed's
-//      predecessor on each of its pixels is the latest earlier claimant, and
-//      a record keeps its distinct predecessors;
+//      predecessors are the earlier claimants of its pixels;
 //   3. order: a ticket order in which every predecessor comes first (the seed
 //      grid sheared so that key = column + K x row grows along every
 //      predecessor pair);
-//   4. replay: warps take tickets, wait for their predecessors, read the masks
-//      of their record's pixels and find the pixels the reference's traversal
+//   4. replay: warps take tickets, wait until their predecessors are settled
+//      (have run, or had their pixel fused and never will), read the masks of
+//      their record's pixels and find the pixels the reference's traversal
 //      fuses — in parallel (a frontier search) where no limit can bind, else
-//      by replaying its depth-first traversal (explicit stack, limits) — mark
-//      them and release their successors; then they compute the fused point
-//      (medians);
+//      by replaying its depth-first traversal (explicit stack, limits) — and
+//      mark them, their own last; then they compute the fused point (medians);
 //   5. compaction of the points in seed order.
 // A traversal only reads or writes the masks of pixels that pass its tests
 // (a pixel that fails them is skipped whether or not it is fused), so two
@@ -63,7 +62,6 @@ constexpr uint32_t kEmpty = 0xffffffffu;
 constexpr uint32_t kOver = 0xfffffffeu;
 constexpr uint32_t kRetry = 0xfffffffdu;  // the record did not fit the pool; built again after it grows
 constexpr int kReplayWarps = 4;        // warps per replay block
-constexpr int kEdgeSh = 1024;          // push-list entries of a record staged in shared memory
 constexpr int kStackSh = 512;          // replay stack entries kept in shared memory per warp
 constexpr int kScanItems = 4096;       // items per scan block (256 threads x 16)
 constexpr unsigned long long kWaitLimitNs = 20ull * 1000 * 1000 * 1000;  // bounded waits: 20 s
@@ -106,17 +104,17 @@ struct FMaps {
   const FView* views;
   const int* ov;          // overlapping_images_, concatenated
   const uint8_t* trav;    // per image: used and not yet fused
-  const float* D;         // depth
-  const float* X;         // inv_P * (col d, row d, d, 1) (fusion.cc:1953-1955)
-  const float* Y;
-  const float* Z;
-  const float* NX;        // inv_R * normal (:1939-1941)
-  const float* NY;
-  const float* NZ;
-  const float* G;         // red-channel gradient (:2007-2021)
+  // Two float4 per pixel, one 32-byte sector: a candidate's test reads both.
+  //   [2 g]     inv_P * (col d, row d, d, 1) (fusion.cc:1953-1955), depth d
+  //   [2 g + 1] inv_R * normal (:1939-1941), red-channel gradient (:2007-2021)
+  const float4* pix;
+  const uint32_t* proj;   // [pixel][deg]: the pixel's place in its overlapping images (pixel index, kNoKey: outside)
+  int deg;                // overlapping images of the image that has most
+  int num_views;
   const uint8_t* rgb;     // W*H*3 per image
   uint8_t* mask;          // fused_pixel_masks_
 };
+constexpr uint32_t kNoKey = 0xffffffffu;
 
 struct FConsts {
   float max_sq_reproj;  // max_squared_reproj_error_ (float)
@@ -135,7 +133,8 @@ struct FImage {
 };
 
 // Record pool of one image. A record (u32 words): cnt, nE, gid[cnt], derr[cnt],
-// eoff[cnt + 1], vid[cnt] (u16), edges[nE bound] (u16).
+// eoff[cnt + 1], vid[cnt] (u16), edges[nE bound] (u8 in records of at most kCap
+// pixels, else u16).
 struct FRecs {
   uint32_t* pool;
   unsigned long long pool_words;
@@ -147,7 +146,7 @@ struct FRecs {
 };
 
 __host__ __device__ inline uint32_t RecWords(uint32_t cnt, uint32_t ebound) {
-  return 2u + 2u * cnt + (cnt + 1u) + (cnt + 1u) / 2u + (ebound + 1u) / 2u;
+  return 2u + 2u * cnt + (cnt + 1u) + (cnt + 1u) / 2u + (cnt <= (uint32_t)kCap ? (ebound + 3u) / 4u : (ebound + 1u) / 2u);
 }
 
 // Bytes of one replay warp's scratch region: stack (u32) | vals (f32) | ids (u32)
@@ -191,33 +190,58 @@ __device__ __forceinline__ bool ProjectPixel(const FView& fu, float x, float y, 
 
 // ---- point maps -------------------------------------------------------------
 __global__ void PointMapKernel(FView v, float R0, float R1, float R2, float R3, float R4, float R5, float R6,
-                               float R7, float R8, const float* __restrict__ normal_in, int with_normal,
-                               int has_color, float* D, float* X, float* Y, float* Z, float* NX, float* NY,
-                               float* NZ, float* G, const uint8_t* __restrict__ rgb) {
+                               float R7, float R8, const float* __restrict__ depth_in,
+                               const float* __restrict__ normal_in, int with_normal, int has_color,
+                               float4* __restrict__ pix, const uint8_t* __restrict__ rgb) {
   const uint32_t plane = (uint32_t)v.W * (uint32_t)v.H;
   for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < plane; p += gridDim.x * blockDim.x) {
     const int row = (int)(p / (uint32_t)v.W), col = (int)(p - (uint32_t)row * (uint32_t)v.W);
-    const uint32_t g = v.base + p;
-    const float d = D[g];
+    const size_t g = (size_t)v.base + p;
+    const float d = depth_in[p];
     const float cd = __fmul_rn((float)col, d), rd = __fmul_rn((float)row, d);
-    X[g] = Dot4p(v.iP, cd, rd, d, 1.0f);
-    Y[g] = Dot4p(v.iP + 4, cd, rd, d, 1.0f);
-    Z[g] = Dot4p(v.iP + 8, cd, rd, d, 1.0f);
+    pix[2 * g] = make_float4(Dot4p(v.iP, cd, rd, d, 1.0f), Dot4p(v.iP + 4, cd, rd, d, 1.0f),
+                             Dot4p(v.iP + 8, cd, rd, d, 1.0f), d);
+    float4 n = make_float4(0.f, 0.f, 0.f, 0.f);
     if (with_normal) {
-      const float n0 = normal_in[p], n1 = normal_in[plane + p], n2 = normal_in[2 * plane + p];
+      const float n0 = normal_in[p], n1 = normal_in[plane + p], n2 = normal_in[2 * (size_t)plane + p];
       // inv_R = R^T: row i of inv_R is column i of R.
-      NX[g] = Dot3(R0, R3, R6, n0, n1, n2);
-      NY[g] = Dot3(R1, R4, R7, n0, n1, n2);
-      NZ[g] = Dot3(R2, R5, R8, n0, n1, n2);
+      n.x = Dot3(R0, R3, R6, n0, n1, n2);
+      n.y = Dot3(R1, R4, R7, n0, n1, n2);
+      n.z = Dot3(R2, R5, R8, n0, n1, n2);
     }
-    float grad = 0.0f;
     if (has_color && col > 1 && col < v.W - 1 && row > 1 && row < v.H - 1) {
       const uint8_t* px = rgb + 3ull * g;
       const float gx = __fdiv_rn((float)((int)px[-3] - (int)px[3]), 255.0f);
       const float gy = __fdiv_rn((float)((int)px[-3 * v.W] - (int)px[3 * v.W]), 255.0f);
-      grad = __fsqrt_rn(__fadd_rn(__fmul_rn(gx, gx), __fmul_rn(gy, gy)));
+      n.w = __fsqrt_rn(__fadd_rn(__fmul_rn(gx, gx), __fmul_rn(gy, gy)));
     }
-    G[g] = grad;
+    pix[2 * g + 1] = n;
+  }
+}
+
+// Where the pixels of image `view` fall in its overlapping images. A closure
+// asks for these places again in every seed that reaches the pixel (some 100
+// seeds in the first image of 11 views): the table replaces two divisions, nine
+// products and the point's read by one word, of ten that lie together.
+__global__ void ProjectTableKernel(FMaps m, int view, uint32_t* __restrict__ proj) {
+  const FView& v = m.views[view];
+  const uint32_t plane = (uint32_t)v.W * (uint32_t)v.H;
+  const int deg = v.ov_end - v.ov_begin;
+  for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < plane; p += gridDim.x * blockDim.x) {
+    const size_t g = (size_t)v.base + p;
+    const float4 x = m.pix[2 * g];
+    const bool ok = ValidDepth(x.w);
+    for (int k = 0; k < m.deg; ++k) {
+      uint32_t e = kNoKey;
+      int row, col;
+      if (ok && k < deg) {
+        const int u = m.ov[v.ov_begin + k];
+        const FView& fu = m.views[u];
+        if (m.trav[u] && ProjectPixel(fu, x.x, x.y, x.z, &row, &col))
+          e = fu.base + (uint32_t)row * (uint32_t)fu.W + (uint32_t)col;
+      }
+      proj[g * (size_t)m.deg + k] = e;
+    }
   }
 }
 
@@ -280,14 +304,9 @@ __device__ __forceinline__ int BuildClosure(const FMaps& m, const FConsts& c, ui
                                             uint32_t* eoff, uint16_t* edges, uint32_t ecap, uint32_t* ne) {
   *ne = 0;
   if (m.mask[sg]) return 0;
-  if (!ValidDepth(m.D[sg])) return 0;
-  const float sx = m.X[sg], sy = m.Y[sg], sz = m.Z[sg];
-  float s0 = 0.f, s1 = 0.f, s2 = 0.f;
-  if (c.with_normal) {
-    s0 = m.NX[sg];
-    s1 = m.NY[sg];
-    s2 = m.NZ[sg];
-  }
+  const float4 sp = m.pix[2 * (size_t)sg], sn = m.pix[2 * (size_t)sg + 1];
+  if (!ValidDepth(sp.w)) return 0;
+  const float sx = sp.x, sy = sp.y, sz = sp.z, s0 = sn.x, s1 = sn.y, s2 = sn.z;
   SeedProj proj;
   proj.Clear();
   set.Clear();
@@ -301,18 +320,18 @@ __device__ __forceinline__ int BuildClosure(const FMaps& m, const FConsts& c, ui
     eoff[i] = e;
     const uint32_t g = gid[i];
     const FView& fv = m.views[vid[i]];
-    const float x = m.X[g], y = m.Y[g], z = m.Z[g];
+    const float4 gp = m.pix[2 * (size_t)g];
     for (int k = fv.ov_begin; k < fv.ov_end; ++k) {
       const int u = m.ov[k];
       if (!m.trav[u]) continue;
       const FView& fu = m.views[u];
       int row, col;
-      if (!ProjectPixel(fu, x, y, z, &row, &col)) continue;
+      if (!ProjectPixel(fu, gp.x, gp.y, gp.z, &row, &col)) continue;
       const uint32_t q = fu.base + (uint32_t)row * (uint32_t)fu.W + (uint32_t)col;
       if (m.mask[q]) continue;
       int j = set.Find(gid, q);
       if (j < 0) {
-        const float dq = m.D[q];
+        const float dq = m.pix[2 * (size_t)q].w;
         if (!ValidDepth(dq)) continue;
         // Reprojection and depth error of the seed point in image u (:1893-1912).
         float pc, pr, pz;
@@ -322,7 +341,8 @@ __device__ __forceinline__ int BuildClosure(const FMaps& m, const FConsts& c, ui
         if (sq > c.max_sq_reproj) continue;
         const float de = __fdiv_rn(fabsf(__fsub_rn(pz, dq)), dq);
         if (de > c.derr_thr) continue;
-        if (c.with_normal && Dot3(s0, s1, s2, m.NX[q], m.NY[q], m.NZ[q]) < c.min_cos) continue;  // :1944-1948
+        const float4 nq = m.pix[2 * (size_t)q + 1];
+        if (c.with_normal && Dot3(s0, s1, s2, nq.x, nq.y, nq.z) < c.min_cos) continue;  // :1944-1948
         if (cnt == cap) return -1;
         j = cnt;
         gid[cnt] = q;
@@ -366,6 +386,7 @@ __device__ bool WriteRecord(const FMaps& m, const FRecs& r, uint32_t seed, const
   uint32_t* eoff = reinterpret_cast<uint32_t*>(rd + cnt);
   uint16_t* rv = reinterpret_cast<uint16_t*>(eoff + cnt + 1);
   uint16_t* edges = rv + 2 * ((cnt + 1) / 2);
+  uint8_t* edges8 = cnt <= kCap ? reinterpret_cast<uint8_t*>(edges) : nullptr;
   for (int i = 0; i < cnt; ++i) {
     rg[i] = gid[i];
     rd[i] = derr[i];
@@ -374,23 +395,26 @@ __device__ bool WriteRecord(const FMaps& m, const FRecs& r, uint32_t seed, const
   uint32_t e = 0;
   if (have_edges) {
     for (int i = 0; i <= cnt; ++i) eoff[i] = leoff[i];
-    for (uint32_t q = 0; q < lne; ++q) edges[q] = ledges[q];
+    for (uint32_t q = 0; q < lne; ++q)
+      if (edges8) edges8[q] = (uint8_t)ledges[q]; else edges[q] = ledges[q];
     e = lne;
   } else {
     for (int i = 0; i < cnt; ++i) {
       eoff[i] = e;
       const uint32_t g = gid[i];
       const FView& fv = m.views[vid[i]];
-      const float x = m.X[g], y = m.Y[g], z = m.Z[g];
+      const float4 gp = m.pix[2 * (size_t)g];
       for (int k = fv.ov_begin; k < fv.ov_end; ++k) {
         const int u = m.ov[k];
         if (!m.trav[u]) continue;
         const FView& fu = m.views[u];
         int row, col;
-        if (!ProjectPixel(fu, x, y, z, &row, &col)) continue;
+        if (!ProjectPixel(fu, gp.x, gp.y, gp.z, &row, &col)) continue;
         const int j = set.Find(gid, fu.base + (uint32_t)row * (uint32_t)fu.W + (uint32_t)col);
         if (j < 0) continue;
-        if (e < ebound) edges[e] = (uint16_t)j;
+        if (e < ebound) {
+          if (edges8) edges8[e] = (uint8_t)j; else edges[e] = (uint16_t)j;
+        }
         ++e;
       }
     }
@@ -415,19 +439,19 @@ __device__ __forceinline__ uint32_t SeedPixel(const FMaps& m, const FImage& im, 
 constexpr int kSetSlots = 2 * kCap;          // hash slots of the closure pass
 constexpr int kBigSetSlots = 2 * 65536;      // hash slots of the overflow pass
 constexpr int kEdgeLocal = 2048;             // push-list entries kept by the closure pass
+// Rejected pixels kept in a closure's hash set: with the round that reaches a
+// bound (32 lanes each) and kCap accepted ones the set is never full.
+constexpr int kMaxRejected = kSetSlots - kCap - 96;
+constexpr uint16_t kReject = 0xffff;
 
 // One warp per seed. The closure under construction lives in shared memory:
 // a hash set of its pixels (key = pixel index, value = node index), the
 // nodes (pixel, image, depth error, point) and their push lists.
 constexpr int kClosureWarps = 4;  // warps (seeds in flight) per closure block
-constexpr uint32_t kNoKey = 0xffffffffu;
-struct ClosureShared;
-
 struct ClosureShared {
   uint32_t keys[kSetSlots];
   uint32_t gid[kCap];
-  uint32_t dpre[kCap + 1];             // push counts of the frontier, prefix-summed
-  uint32_t ecnt[kCap];
+  float seed[3][32];                   // the seed's column, row and depth in images 0..31
   uint16_t kidx[kSetSlots];
   uint16_t vid[kCap];
 };
@@ -435,58 +459,52 @@ struct ClosureShared {
 // A closure warp's global staging (L2-resident for the whole grid): the push
 // lists, their offsets and the depth errors, each written once and read when
 // the record is written.
-constexpr size_t kStageEoff = 2u * (size_t)kEdgeLocal;                  // u32[kCap + 1]
+constexpr size_t kStageEoff = (size_t)kEdgeLocal;                       // u32[kCap + 1]
 constexpr size_t kStageDerr = kStageEoff + 4u * ((size_t)kCap + 1u);   // f32[kCap]
 constexpr size_t kStageBytes = (kStageDerr + 4u * (size_t)kCap + 15u) & ~(size_t)15u;
-
-// Exclusive prefix sum over a[lo..hi) into out[lo..hi], out[lo] = base.
-__device__ __forceinline__ void WarpPrefix(const uint32_t* a, uint32_t* out, int lo, int hi, uint32_t base,
-                                           int lane) {
-  uint32_t carry = base;
-  for (int i0 = lo; i0 < hi; i0 += 32) {
-    const int i = i0 + lane;
-    const uint32_t x = i < hi ? a[i] : 0u;
-    uint32_t incl = x;
-    for (int o = 1; o < 32; o <<= 1) {
-      const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
-      if (lane >= o) incl += y;
-    }
-    if (i < hi) out[i] = carry + incl - x;
-    carry += __shfl_sync(0xffffffffu, incl, 31);
-  }
-  if (lane == 0) out[hi] = carry;
-  __syncwarp();
-}
 
 constexpr size_t kClosureSmem = sizeof(ClosureShared) * kClosureWarps;
 
 // `stage`: kStageBytes per warp of the grid (global memory; tens of MB for the
-// whole grid, so they stay in L2).
+// whole grid, so they stay in L2). kTable: the projections come from m.proj.
+// The kernel is bound by the latency of its gathers (a frontier pixel's places, a
+// candidate's sector and mask), so these are few and independent, the next
+// round's places are read ahead, and the seed's own projections, which every
+// candidate's test needs, are computed once per image. Measured on the first
+// image of 11 views 1600x1200: 26.1 ms (60.9 with eight separate maps, every
+// projection in place and each candidate read whatever its distance). Now its
+// instructions bound it: 67 % of the issue slots, 17 of 32 lanes.
+template <bool kTable>
 __global__ void __launch_bounds__(32 * kClosureWarps) ClosureKernel(FMaps m, FConsts c, FImage im, FRecs r,
                                                                     int only_retry, uint8_t* stage) {
   extern __shared__ __align__(16) unsigned char closure_smem[];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   ClosureShared& sh = reinterpret_cast<ClosureShared*>(closure_smem)[w];
   uint8_t* const wstage = stage + ((size_t)blockIdx.x * kClosureWarps + w) * kStageBytes;
-  uint16_t* const edges = reinterpret_cast<uint16_t*>(wstage);
+  uint8_t* const edges = wstage;
   uint32_t* const eoff = reinterpret_cast<uint32_t*>(wstage + kStageEoff);
   float* const derr = reinterpret_cast<float*>(wstage + kStageDerr);
   const unsigned lt = (1u << lane) - 1u;
+  const int D = m.deg > 0 ? m.deg : 1;
+  const int q32 = 32 / D, r32 = 32 - q32 * D;
   for (uint32_t s = blockIdx.x * kClosureWarps + w; s < im.nseeds; s += gridDim.x * kClosureWarps) {
     if (only_retry && r.rec_off[s] != kRetry) continue;
     const uint32_t sg = SeedPixel(m, im, s);
-    if (m.mask[sg] || !ValidDepth(m.D[sg])) {
+    const float4 sp = m.pix[2 * (size_t)sg];
+    if (m.mask[sg] || !ValidDepth(sp.w)) {
       if (lane == 0) r.rec_off[s] = kEmpty;
       continue;
     }
-    const float sx = m.X[sg], sy = m.Y[sg], sz = m.Z[sg];
-    float s0 = 0.f, s1 = 0.f, s2 = 0.f;
-    if (c.with_normal) {
-      s0 = m.NX[sg];
-      s1 = m.NY[sg];
-      s2 = m.NZ[sg];
-    }
+    const float4 sn = m.pix[2 * (size_t)sg + 1];
     for (int h = lane; h < kSetSlots; h += 32) sh.keys[h] = kNoKey;
+    if (lane < m.num_views && m.trav[lane]) {
+      const FView& fu = m.views[lane];
+      const float p0 = Dot4p(fu.P, sp.x, sp.y, sp.z, 1.0f), p1 = Dot4p(fu.P + 4, sp.x, sp.y, sp.z, 1.0f),
+                  p2 = Dot4p(fu.P + 8, sp.x, sp.y, sp.z, 1.0f);
+      sh.seed[0][lane] = __fdiv_rn(p0, p2);
+      sh.seed[1][lane] = __fdiv_rn(p1, p2);
+      sh.seed[2][lane] = p2;
+    }
     __syncwarp();
     if (lane == 0) {
       const uint32_t h = ((sg * 0x9E3779B1u) >> 7) & (uint32_t)(kSetSlots - 1);
@@ -498,80 +516,102 @@ __global__ void __launch_bounds__(32 * kClosureWarps) ClosureKernel(FMaps m, FCo
       eoff[0] = 0;
     }
     __syncwarp();
-    int cnt = 1, head = 0;
+    int cnt = 1, head = 0, rejected = 0;
     uint32_t ecur = 0;
     bool over = false;
     // Breadth-first waves: every (frontier pixel, overlapping image) pair is
     // one lane's candidate; pairs run in pixel-major, image order, so the push
-    // lists come out in the reference's order.
-    while (head < cnt && !over) {
+    // lists come out in the reference's order. Every pixel counts D pairs; those
+    // beyond its image's list are empty.
+    while (m.deg > 0 && head < cnt && !over) {
       const int tail = cnt;
-      for (int i = head + lane; i < tail; i += 32) {
-        const FView& fv = m.views[sh.vid[i]];
-        sh.ecnt[i] = (uint32_t)(fv.ov_end - fv.ov_begin);
-      }
-      __syncwarp();
-      WarpPrefix(sh.ecnt, sh.dpre, head, tail, 0u, lane);
-      for (int i = head + lane; i < tail; i += 32) sh.ecnt[i] = 0;
-      __syncwarp();
-      const uint32_t P = sh.dpre[tail];
-      for (uint32_t p0 = 0; p0 < P && !over; p0 += 32) {
-        const uint32_t p = p0 + lane;
-        // 0 none, 1 found/duplicate (read kidx[h] later), 2 owner of a new node
-        int kind = 0, i = 0, u = 0;
-        uint32_t h = 0, q = 0;
+      int i = head + lane / D, k = lane - (lane / D) * D;
+      uint32_t place = kNoKey;
+      if (kTable && i < tail) place = m.proj[(size_t)sh.gid[i] * m.deg + k];
+      while (__any_sync(0xffffffffu, i < tail)) {
+        // The next round's pair and place.
+        int ni = i + q32, nk = k + r32;
+        if (nk >= D) { nk -= D; ++ni; }
+        uint32_t nplace = kNoKey;
+        if (kTable && ni < tail) nplace = m.proj[(size_t)sh.gid[ni] * m.deg + nk];
+        // 0 none, 1 found/duplicate (read kidx[h] later), 2 owner of a new node, 3
+        // of a pixel that was read and rejected (kept too, so that it is read once)
+        int kind = 0, u = 0;
+        uint32_t h = 0, q = kNoKey;
         float de = 0.f;
-        if (p < P) {
-          int lo = head, hi = tail - 1;  // the frontier pixel whose pushes hold p
-          while (lo < hi) {
-            const int mid = (lo + hi + 1) >> 1;
-            if (sh.dpre[mid] <= p) lo = mid; else hi = mid - 1;
-          }
-          i = lo;
+        int row = 0, col = 0;
+        if (kTable) {
+          q = place;
+        } else if (i < tail) {
           const FView& fv = m.views[sh.vid[i]];
-          u = m.ov[fv.ov_begin + (int)(p - sh.dpre[i])];
-          int row, col;
-          const uint32_t gi = sh.gid[i];
-          if (m.trav[u] && ProjectPixel(m.views[u], m.X[gi], m.Y[gi], m.Z[gi], &row, &col)) {
+          if (fv.ov_begin + k < fv.ov_end) {
+            u = m.ov[fv.ov_begin + k];
             const FView& fu = m.views[u];
-            q = fu.base + (uint32_t)row * (uint32_t)fu.W + (uint32_t)col;
-            if (!m.mask[q]) {
-              h = ((q * 0x9E3779B1u) >> 7) & (uint32_t)(kSetSlots - 1);
-              const volatile uint32_t* vkeys = sh.keys;  // other lanes insert concurrently
-              uint32_t key;
-              while ((key = vkeys[h]) != kNoKey && key != q) h = (h + 1) & (uint32_t)(kSetSlots - 1);
-              if (key == q) {
-                kind = 1;
-              } else {
-                const float dq = m.D[q];
-                bool ok = ValidDepth(dq);
-                if (ok) {
-                  const float p0 = Dot4p(fu.P, sx, sy, sz, 1.0f), p1 = Dot4p(fu.P + 4, sx, sy, sz, 1.0f),
-                              p2 = Dot4p(fu.P + 8, sx, sy, sz, 1.0f);
-                  const float cdiff = __fsub_rn(__fdiv_rn(p0, p2), (float)col);
-                  const float rdiff = __fsub_rn(__fdiv_rn(p1, p2), (float)row);
-                  const float sq = __fadd_rn(__fmul_rn(cdiff, cdiff), __fmul_rn(rdiff, rdiff));
-                  de = __fdiv_rn(fabsf(__fsub_rn(p2, dq)), dq);
-                  ok = !(sq > c.max_sq_reproj) && !(de > c.derr_thr);
-                  if (ok && c.with_normal) ok = !(Dot3(s0, s1, s2, m.NX[q], m.NY[q], m.NZ[q]) < c.min_cos);
-                }
-                if (ok) {  // claim a slot; a lane of this round may hold the same pixel
-                  for (;;) {
-                    const uint32_t old = atomicCAS(&sh.keys[h], kNoKey, q);
-                    if (old == kNoKey) { kind = 2; break; }
-                    if (old == q) { kind = 1; break; }
-                    h = (h + 1) & (uint32_t)(kSetSlots - 1);
-                  }
-                }
+            const float4 gp = m.pix[2 * (size_t)sh.gid[i]];
+            if (m.trav[u] && ProjectPixel(fu, gp.x, gp.y, gp.z, &row, &col))
+              q = fu.base + (uint32_t)row * (uint32_t)fu.W + (uint32_t)col;
+          }
+        }
+        if (q != kNoKey) {
+          h = ((q * 0x9E3779B1u) >> 7) & (uint32_t)(kSetSlots - 1);
+          const volatile uint32_t* vkeys = sh.keys;  // other lanes insert concurrently
+          uint32_t key;
+          while ((key = vkeys[h]) != kNoKey && key != q) h = (h + 1) & (uint32_t)(kSetSlots - 1);
+          if (key == q) {
+            kind = 1;
+          } else {
+            // The reprojection test first: it needs no read, and most of the
+            // pixels that fail fail it.
+            if (kTable) u = m.ov[m.views[sh.vid[i]].ov_begin + k];
+            const FView& fu = m.views[u];
+            if (kTable) {
+              const uint32_t px = q - fu.base;
+              row = (int)__fmul_rn((float)px, __frcp_rn((float)fu.W));  // at most one off
+              col = (int)px - row * fu.W;
+              if (col < 0) { col += fu.W; --row; }
+              if (col >= fu.W) { col -= fu.W; ++row; }
+            }
+            float pc, pr, pz;
+            if (u < 32) {
+              pc = sh.seed[0][u];
+              pr = sh.seed[1][u];
+              pz = sh.seed[2][u];
+            } else {
+              const float p0 = Dot4p(fu.P, sp.x, sp.y, sp.z, 1.0f), p1 = Dot4p(fu.P + 4, sp.x, sp.y, sp.z, 1.0f);
+              pz = Dot4p(fu.P + 8, sp.x, sp.y, sp.z, 1.0f);
+              pc = __fdiv_rn(p0, pz);
+              pr = __fdiv_rn(p1, pz);
+            }
+            const float cdiff = __fsub_rn(pc, (float)col), rdiff = __fsub_rn(pr, (float)row);
+            const float sq = __fadd_rn(__fmul_rn(cdiff, cdiff), __fmul_rn(rdiff, rdiff));
+            const bool close = m.trav[u] && !(sq > c.max_sq_reproj);
+            bool ok = close;
+            if (close) {
+              const uint8_t fused = m.mask[q];
+              const float4 xq = m.pix[2 * (size_t)q], nq = m.pix[2 * (size_t)q + 1];
+              ok = !fused && ValidDepth(xq.w);
+              if (ok) {
+                de = __fdiv_rn(fabsf(__fsub_rn(pz, xq.w)), xq.w);
+                ok = !(de > c.derr_thr);
               }
+              if (ok && c.with_normal) ok = !(Dot3(sn.x, sn.y, sn.z, nq.x, nq.y, nq.z) < c.min_cos);
+            }
+            if (ok || (close && rejected < kMaxRejected)) {  // claim a slot; a lane of this round may hold the same pixel
+              for (;;) {
+                const uint32_t old = atomicCAS(&sh.keys[h], kNoKey, q);
+                if (old == kNoKey) { kind = ok ? 2 : 3; break; }
+                if (old == q) { kind = 1; break; }
+                h = (h + 1) & (uint32_t)(kSetSlots - 1);
+              }
+              if (kind == 3) sh.kidx[h] = kReject;
             }
           }
         }
         __syncwarp();
-        const unsigned own = __ballot_sync(0xffffffffu, kind == 2);
+        const unsigned fresh = __ballot_sync(0xffffffffu, kind == 2);
         int j = -1;
         if (kind == 2) {
-          j = cnt + __popc(own & lt);
+          j = cnt + __popc(fresh & lt);
           if (j < im.cap) {
             sh.kidx[h] = (uint16_t)j;
             sh.gid[j] = q;
@@ -579,23 +619,32 @@ __global__ void __launch_bounds__(32 * kClosureWarps) ClosureKernel(FMaps m, FCo
             derr[j] = de;
           }
         }
-        cnt += __popc(own);
+        cnt += __popc(fresh);
+        rejected += __popc(__ballot_sync(0xffffffffu, kind == 3));
         if (cnt > im.cap) over = true;
         __syncwarp();
-        if (kind == 1) j = sh.kidx[h];
+        if (kind == 1) {
+          const uint32_t e = sh.kidx[h];
+          j = e == kReject ? -1 : (int)e;
+        }
         const unsigned val = __ballot_sync(0xffffffffu, j >= 0);
         const uint32_t at = ecur + (uint32_t)__popc(val & lt);
-        if (j >= 0 && !over) {
-          if (at < (uint32_t)kEdgeLocal) edges[at] = (uint16_t)j;
-          atomicAdd(&sh.ecnt[i], 1u);
+        if (!over) {
+          if (i < tail && k == 0) eoff[i] = at;
+          if (j >= 0 && at < (uint32_t)kEdgeLocal) edges[at] = (uint8_t)j;
         }
         ecur += (uint32_t)__popc(val);
         if (ecur > (uint32_t)kEdgeLocal) over = true;
         __syncwarp();
+        if (over) break;
+        i = ni;
+        k = nk;
+        place = nplace;
       }
-      if (!over) WarpPrefix(sh.ecnt, eoff, head, tail, eoff[head], lane);
       head = tail;
     }
+    if (!over && lane == 0) eoff[cnt] = ecur;
+    __syncwarp();
     if (over) {
       if (lane == 0) {
         r.rec_off[s] = kOver;
@@ -622,14 +671,15 @@ __global__ void __launch_bounds__(32 * kClosureWarps) ClosureKernel(FMaps m, FCo
     float* rd = reinterpret_cast<float*>(rg + cnt);
     uint32_t* reo = reinterpret_cast<uint32_t*>(rd + cnt);
     uint16_t* rv = reinterpret_cast<uint16_t*>(reo + cnt + 1);
-    uint16_t* redg = rv + 2 * ((cnt + 1) / 2);
+    uint8_t* redg = reinterpret_cast<uint8_t*>(rv + 2 * ((cnt + 1) / 2));
     for (int k = lane; k < cnt; k += 32) {
       rg[k] = sh.gid[k];
       rd[k] = derr[k];
       rv[k] = sh.vid[k];
     }
     for (int k = lane; k <= cnt; k += 32) reo[k] = eoff[k];
-    for (uint32_t k = lane; k < ne; k += 32) redg[k] = edges[k];
+    for (uint32_t k = lane; k < (ne + 3u) / 4u; k += 32)
+      reinterpret_cast<uint32_t*>(redg)[k] = reinterpret_cast<const uint32_t*>(edges)[k];
     if (lane == 0) {
       rec[0] = (uint32_t)cnt;
       rec[1] = ne;
@@ -672,7 +722,8 @@ struct RecView {
   const float* derr;
   const uint32_t* eoff;
   const uint16_t* vid;
-  const uint16_t* edges;
+  const uint16_t* edges;  // of a record over kCap pixels, else edges8
+  const uint8_t* edges8;
 };
 
 __device__ __forceinline__ RecView OpenRecord(uint32_t* pool, uint32_t off) {
@@ -685,6 +736,7 @@ __device__ __forceinline__ RecView OpenRecord(uint32_t* pool, uint32_t off) {
   v.eoff = rec + 2 + 2 * v.cnt;
   v.vid = reinterpret_cast<const uint16_t*>(v.eoff + v.cnt + 1);
   v.edges = v.vid + 2 * ((v.cnt + 1) / 2);
+  v.edges8 = reinterpret_cast<const uint8_t*>(v.edges);
   return v;
 }
 
@@ -731,82 +783,117 @@ struct FPreds {
   const uint32_t* claim_list;
 };
 constexpr uint32_t kWalk = 0xffffffffu;
-constexpr int kPredSlots = 512;  // hash slots of a seed's distinct predecessors
-constexpr int kPredMost = 384;   // with more of them the replay walks the claims
+constexpr int kFarSlots = 128;   // hash slots of the distinct predecessors outside the window
+constexpr int kFarMost = 64;     // with more of them the replay walks the claims
 
+// One warp per seed. Nearly all predecessors lie in the seed grid's 8 rows x 32
+// columns up to the seed (a record's pixels are within the reprojection radius of
+// its seed's point), so they are collected as bits of 8 words, each set once: a
+// claim whose bit is set costs a read and a test. The others go through a small
+// hash set. Measured with the claim kernels on the first image of 11 views
+// 1600x1200 (some 640 claims a seed): 9.2 ms; 22 with one hash set for all.
 __global__ void __launch_bounds__(256) PredKernel(FMaps m, FImage im, FRecs r, FPreds pr, int* shear) {
-  __shared__ uint32_t keys_all[8][kPredSlots];
+  __shared__ uint32_t far_all[8][kFarSlots];
+  __shared__ uint32_t near_all[8][8];
   __shared__ uint32_t count_all[8];
   const uint32_t s = (uint32_t)(((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-  const uint32_t lane = threadIdx.x & 31;
-  uint32_t* keys = keys_all[threadIdx.x >> 5];
-  volatile uint32_t* count = count_all + (threadIdx.x >> 5);
+  const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  uint32_t* keys = far_all[w];
+  uint32_t* near = near_all[w];
+  volatile uint32_t* count = count_all + w;
   if (s >= im.nseeds) return;
   const uint32_t off = r.rec_off[s];
   if (off >= kRetry) return;
   const RecView v = OpenRecord(r.pool, off);
-  for (int i = lane; i < kPredSlots; i += 32) keys[i] = kNoKey;
+  for (int i = lane; i < kFarSlots; i += 32) keys[i] = kNoKey;
+  if (lane < 8) near[lane] = 0u;
   if (lane == 0) *count = 0;
   __syncwarp();
+  const uint32_t Cs = (uint32_t)im.Cs;
+  const float inv_cs = 1.0f / (float)im.Cs;
+  const volatile uint32_t* vnear = near;
+  const volatile uint32_t* vk = keys;
+  auto add = [&](uint32_t cl) {
+    if (cl >= s) return;
+    // s - cl = rows * Cs + columns with columns in [-16, 15].
+    const uint32_t d = s - cl + 16u;
+    const uint32_t row = (uint32_t)((float)d * inv_cs);
+    const uint32_t bit = d - row * Cs;  // wraps to a large value where row was rounded up
+    if (Cs >= 32u && row < 8u && bit < 32u) {
+      if (!((vnear[row] >> bit) & 1u)) atomicOr(near + row, 1u << bit);
+      return;
+    }
+    if (*count > (uint32_t)kFarMost) return;  // the table never fills up
+    uint32_t h = (cl * 0x9E3779B1u) >> 25;  // 128 slots
+    for (;;) {
+      uint32_t key = vk[h];
+      if (key == kNoKey) key = atomicCAS(keys + h, kNoKey, cl);
+      if (key == kNoKey) { atomicAdd(count_all + w, 1u); return; }
+      if (key == cl) return;
+      h = (h + 1) & (uint32_t)(kFarSlots - 1);
+    }
+  };
   for (uint32_t k = lane; k < v.cnt; k += 32) {
     const uint32_t g = v.gid[k];
-    for (uint32_t q = pr.claim_off[g], end = pr.claim_off[g + 1]; q < end; ++q) {
-      const uint32_t cl = pr.claim_list[q];
-      if (cl >= s || *count > (uint32_t)kPredMost) continue;  // the table never fills up
-      uint32_t h = (cl * 0x9E3779B1u) >> 23;  // 512 slots
-      const volatile uint32_t* vk = keys;
-      for (;;) {
-        uint32_t key = vk[h];
-        if (key == kNoKey) key = atomicCAS(keys + h, kNoKey, cl);
-        if (key == kNoKey) { atomicAdd(count_all + (threadIdx.x >> 5), 1u); break; }
-        if (key == cl) break;
-        h = (h + 1) & (uint32_t)(kPredSlots - 1);
-      }
+    const uint32_t end = pr.claim_off[g + 1];
+    for (uint32_t q = pr.claim_off[g]; q < end; q += 4) {  // four claims in flight
+      const uint32_t c0 = pr.claim_list[q];
+      const uint32_t c1 = q + 1 < end ? pr.claim_list[q + 1] : s;
+      const uint32_t c2 = q + 2 < end ? pr.claim_list[q + 2] : s;
+      const uint32_t c3 = q + 3 < end ? pr.claim_list[q + 3] : s;
+      add(c0);
+      add(c1);
+      add(c2);
+      add(c3);
     }
   }
   __syncwarp();
-  const uint32_t n = *count;
+  const uint32_t nfar = *count;
+  uint32_t n = nfar;
+  for (int i = 0; i < 8; ++i) n += (uint32_t)__popc(near[i]);
   unsigned long long at = 0;
-  if (lane == 0 && n > 0 && n <= (uint32_t)kPredMost) at = atomicAdd(pr.used, (unsigned long long)n);
+  const bool many = nfar > (uint32_t)kFarMost;
+  if (lane == 0 && n > 0 && !many) at = atomicAdd(pr.used, (unsigned long long)n);
   at = __shfl_sync(0xffffffffu, at, 0);
-  const bool walk = n > (uint32_t)kPredMost || at + n > pr.cap;
+  const bool walk = many || at + n > pr.cap;
   if (lane == 0) {
     pr.off[s] = (uint32_t)at;
     pr.cnt[s] = walk ? kWalk : n;
   }
-  // The list, and what the distinct predecessors need of the shear (with more
-  // than kPredMost, of every claim).
-  const int Cs = im.Cs;
-  const int is = (int)(s / (uint32_t)Cs), js = (int)(s - (uint32_t)is * (uint32_t)Cs);
+  // The list, and what the predecessors need of the shear (with too many far
+  // ones, of every claim).
+  const int is = (int)(s / Cs), js = (int)(s - (uint32_t)is * Cs);
   int need = 1;
   auto shear_of = [&](uint32_t p) {
-    const int ip = (int)(p / (uint32_t)Cs), jp = (int)(p - (uint32_t)ip * (uint32_t)Cs);
+    const int ip = (int)(p / Cs), jp = (int)(p - (uint32_t)ip * Cs);
     if (ip < is) {
       const int num = jp - js, den = is - ip;
       const int fl = num >= 0 ? num / den : -((-num + den - 1) / den);
       need = max(need, fl + 1);
     }
   };
-  if (n > (uint32_t)kPredMost) {
+  if (many) {
     for (uint32_t k = lane; k < v.cnt; k += 32) {
       const uint32_t g = v.gid[k];
       for (uint32_t q = pr.claim_off[g], end = pr.claim_off[g + 1]; q < end; ++q)
         if (pr.claim_list[q] < s) shear_of(pr.claim_list[q]);
     }
-  } else if (n > 0) {
+  } else {
     uint32_t pos = 0;
-    for (int i0 = 0; i0 < kPredSlots; i0 += 32) {
-      const uint32_t p = keys[i0 + lane];
-      const unsigned has = __ballot_sync(0xffffffffu, p != kNoKey);
-      if (p != kNoKey) {
+    auto put = [&](bool has, uint32_t p) {
+      const unsigned who = __ballot_sync(0xffffffffu, has);
+      if (has) {
         shear_of(p);
-        if (!walk) pr.list[at + pos + (uint32_t)__popc(has & ((1u << lane) - 1u))] = SeedPixel(m, im, p);
+        if (!walk) pr.list[at + pos + (uint32_t)__popc(who & ((1u << lane) - 1u))] = SeedPixel(m, im, p);
       }
-      pos += (uint32_t)__popc(has);
-    }
+      pos += (uint32_t)__popc(who);
+    };
+    for (uint32_t row = 0; row < 8; ++row) put((near[row] >> lane) & 1u, s + 16u - row * Cs - lane);
+    if (nfar > 0)
+      for (int i0 = 0; i0 < kFarSlots; i0 += 32) put(keys[i0 + lane] != kNoKey, keys[i0 + lane]);
   }
   for (int o = 16; o > 0; o >>= 1) need = max(need, __shfl_xor_sync(0xffffffffu, need, o));
-  if (lane == 0 && need > 1) atomicMax(shear, min(need, Cs));
+  if (lane == 0 && need > 1) atomicMax(shear, min(need, im.Cs));
 }
 
 // ---- ticket order ------------------------------------------------------------
@@ -858,20 +945,20 @@ struct FReplay {
   long long withhold;         // test hook: this seed's successors are never released (-1: none, -2: all)
 };
 
-struct WarpShared {
+struct alignas(16) WarpShared {
+  alignas(16) float vals[kCap];  // read as uint4 by WarpMedian64
   uint32_t stack[kStackSh];
-  uint32_t gid[kCap];        // the record, staged before the wait
-  uint32_t eoff[kCap + 1];
-  float vals[kCap];
+  uint32_t gid[kCap];        // the record's pixels, staged before the wait
   uint32_t ids[kCap];
-  uint16_t edges[kEdgeSh];
   uint16_t acc[kCap];
   uint8_t flags[kCap];
-  uint32_t bits[kCap / 32];  // reachability search: pixels fused before or reached
-  int qtail;
+  uint8_t node[kCap];        // the open pixels (not fused before the wait) in the record
+  uint8_t place[kCap];       // and a record pixel's place among them
+  uint32_t images[32];       // images of the cluster (the first 1024)
   float med[2];
   int nacc;
 };
+constexpr int kOpenMost = 128;  // open pixels searched in registers
 
 __device__ __forceinline__ uint32_t LoadMask(const uint8_t* p) {
   uint32_t v;
@@ -907,19 +994,59 @@ __device__ float WarpMedian(const float* vals, int n, float* med, int lane) {
   return r;
 }
 
-// Waits until the masks of the seed pixels that the lanes hold (`pending` lanes)
-// are set, or the seed's own pixel is (true: another seed fused it, nothing is
-// left to do). A short spin, then a back-off; bounded in time (status bit on
-// timeout). Called by the whole warp.
-__device__ __forceinline__ bool WaitSettled(const uint8_t* mask, uint32_t own, uint32_t pixel, bool pending,
-                                            uint32_t* stats, unsigned long long limit_ns) {
+// The same for n <= 64 values, lane l holding values l and l + 32 (anything
+// beyond n; `vals`: 64 words on a 16-byte boundary): each lane ranks its two against all keys, read four at a time.
+__device__ __forceinline__ float WarpMedian64(float a, float b, int n, float* vals, float* med, int lane) {
+  uint32_t* keys = reinterpret_cast<uint32_t*>(vals);
+  const uint32_t ka = lane < n ? FKey(a) : 0xffffffffu, kb = lane + 32 < n ? FKey(b) : 0xffffffffu;
+  keys[lane] = ka;
+  keys[lane + 32] = kb;
+  __syncwarp();
+  // Keys below, and keys equal and before (ties are broken by position). The
+  // padding is the largest key and comes last.
+  int ra = 0, rb = 0;
+  for (int j = 0; j < n; j += 4) {
+    const uint4 k = *reinterpret_cast<const uint4*>(keys + j);
+    ra += (k.x < ka || (k.x == ka && j < lane)) + (k.y < ka || (k.y == ka && j + 1 < lane)) +
+          (k.z < ka || (k.z == ka && j + 2 < lane)) + (k.w < ka || (k.w == ka && j + 3 < lane));
+    if (n > 32)
+      rb += (k.x < kb || (k.x == kb && j < lane + 32)) + (k.y < kb || (k.y == kb && j + 1 < lane + 32)) +
+            (k.z < kb || (k.z == kb && j + 2 < lane + 32)) + (k.w < kb || (k.w == kb && j + 3 < lane + 32));
+  }
+  const int mid = n / 2;
+  if (lane < n) {
+    if (ra == mid) med[0] = a;
+    if ((n & 1) == 0 && ra == mid - 1) med[1] = a;
+  }
+  if (lane + 32 < n) {
+    if (rb == mid) med[0] = b;
+    if ((n & 1) == 0 && rb == mid - 1) med[1] = b;
+  }
+  __syncwarp();
+  const float r = (n & 1) ? med[0] : __fdiv_rn(__fadd_rn(med[0], med[1]), 2.0f);
+  __syncwarp();
+  return r;
+}
+
+// Waits until the masks of the seed pixels that the lanes hold (bit i of `pending`:
+// pixel[i]) are set, or the seed's own pixel is (true: another seed fused it,
+// nothing is left to do). A short spin, then a back-off; bounded in time (status
+// bit on timeout). Called by the whole warp.
+__device__ __forceinline__ bool WaitSettled(const uint8_t* mask, uint32_t own, const uint32_t pixel[4],
+                                            uint32_t pending, uint32_t* stats, unsigned long long limit_ns) {
   const int lane = threadIdx.x & 31;
   unsigned long long t0 = 0;
   for (uint32_t it = 0;; ++it) {
+    uint32_t set[4] = {0u, 0u, 0u, 0u};
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      if ((pending >> i) & 1u) set[i] = LoadMask(mask + pixel[i]);
     bool fused = false;
-    if (pending && LoadMask(mask + pixel)) pending = false;
     if (lane == 31) fused = LoadMask(mask + own) != 0u;
-    const unsigned open = __ballot_sync(0xffffffffu, pending);
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      if (set[i]) pending &= ~(1u << i);
+    const unsigned open = __ballot_sync(0xffffffffu, pending != 0u);
     if (__any_sync(0xffffffffu, fused)) return true;
     if (!open) return false;
     if (it < 16) continue;
@@ -941,8 +1068,9 @@ __device__ __forceinline__ bool WaitSettled(const uint8_t* mask, uint32_t own, u
 // are flagged and listed in acc in the order the reference fuses them. A
 // pushed pixel that is already fused would be skipped when popped, so it is
 // not pushed. Returns the number accepted.
+template <typename Edge>
 __device__ int SeqTraversal(uint8_t* __restrict__ flags, uint32_t* __restrict__ stack, uint16_t* __restrict__ acc,
-                            const uint32_t* __restrict__ reoff, const uint16_t* __restrict__ redges, int max_pix,
+                            const uint32_t* __restrict__ reoff, const Edge* __restrict__ redges, int max_pix,
                             int max_depth) {
   int nacc = 0, top = 0;
   if (!flags[0]) stack[top++] = 0u;
@@ -975,7 +1103,14 @@ __device__ int SeqTraversal(uint8_t* __restrict__ flags, uint32_t* __restrict__ 
   return nacc;
 }
 
-__global__ void __launch_bounds__(32 * kReplayWarps) ReplayKernel(FMaps m, FConsts c, FRecs r, FReplay rp) {
+// Bound by its chain of dependent seeds (the first image of 11 views 1600x1200: 2,759
+// run one after another, each fusing some 36 pixels): what counts is the time
+// from a predecessor's mark to this seed's, so everything that does not depend on
+// the masks is done before the wait. 16 to 20 warps an SM are enough, more only
+// share the issue slots with the seeds on the chain. Measured for that image:
+// 65.6 ms when every earlier claimant's ticket was waited for and the search read
+// its push lists after the wait, now 27.6.
+__global__ void __launch_bounds__(32 * kReplayWarps, 4) ReplayKernel(FMaps m, FConsts c, FRecs r, FReplay rp) {
   __shared__ WarpShared shm[kReplayWarps];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   WarpShared& sh = shm[w];
@@ -1025,17 +1160,63 @@ __global__ void __launch_bounds__(32 * kReplayWarps) ReplayKernel(FMaps m, FCons
     }
     const uint32_t* rgid = v.gid;
     const uint32_t* reoff = v.eoff;
-    const uint16_t* redges = v.edges;
+    // A record over kCap pixels has 16-bit push lists.
+    const bool wide = cnt > kCap;
+    const uint8_t* redges = v.edges8;
+    // Before the wait: the pixels that earlier seeds have not fused yet (marks
+    // are never taken back), and their push lists as bits. Lane l holds the rows
+    // of open pixels l, l + 32, l + 64 and l + 96, so that a step of the search
+    // after the wait, which every successor waits for, is four tests and four
+    // warp-wide ORs.
+    int nopen = kOpenMost + 1;
+    uint32_t rows[4][4], open_gid[4];
     if (node_sh) {
-      for (int k = lane; k < cnt; k += 32) sh.gid[k] = v.gid[k];
-      for (int k = lane; k <= cnt; k += 32) sh.eoff[k] = v.eoff[k];
+      nopen = 0;
+      for (int k0 = 0; k0 < cnt; k0 += 32) {
+        const int k = k0 + lane;
+        bool is_open = false;
+        if (k < cnt) {
+          const uint32_t g = v.gid[k];
+          sh.gid[k] = g;
+          const uint8_t f = __ldcg(m.mask + g);
+          flags[k] = f;
+          is_open = f == 0;
+        }
+        const unsigned who = __ballot_sync(0xffffffffu, is_open);
+        if (is_open) {
+          const int at = nopen + __popc(who & ((1u << lane) - 1u));
+          sh.node[at] = (uint8_t)k;
+          sh.place[k] = (uint8_t)at;
+        }
+        nopen += __popc(who);
+      }
+      __syncwarp();
+      if (flags[0]) continue;  // fused by an earlier seed
       rgid = sh.gid;
-      reoff = sh.eoff;
-      if (v.ne <= (uint32_t)kEdgeSh) {
-        for (uint32_t k = lane; k < v.ne; k += 32) sh.edges[k] = v.edges[k];
-        redges = sh.edges;
+      if (nopen <= kOpenMost) {
+#pragma unroll
+        for (int a = 0; a < 4; ++a) {
+          rows[a][0] = rows[a][1] = rows[a][2] = rows[a][3] = 0u;
+          open_gid[a] = own;
+          const int i = lane + 32 * a;
+          if (i >= nopen) continue;
+          const int k = sh.node[i];
+          open_gid[a] = sh.gid[k];
+          for (uint32_t q = reoff[k], qe = reoff[k + 1]; q < qe; ++q) {
+            const uint32_t j = redges[q];
+            if (flags[j]) continue;
+            const uint32_t at = sh.place[j], bit = 1u << (at & 31u), word = at >> 5;
+#pragma unroll
+            for (uint32_t t = 0; t < 4; ++t) rows[a][t] |= word == t ? bit : 0u;
+          }
+        }
       }
     }
+    const bool in_regs = nopen <= kOpenMost;
+    auto traverse = [&]() -> int {
+      return wide ? SeqTraversal(flags, stack, acc, reoff, v.edges, c.max_pix, c.max_depth)
+                  : SeqTraversal(flags, stack, acc, reoff, redges, c.max_pix, c.max_depth);
+    };
     unsigned long long tw0 = 0;
     if (rp.times) tw0 = GlobalTimer();
     // Wait for the predecessors (every earlier seed that may touch these
@@ -1047,9 +1228,15 @@ __global__ void __launch_bounds__(32 * kReplayWarps) ReplayKernel(FMaps m, FCons
     const uint32_t npred = rp.preds.cnt[s];
     if (npred != kWalk) {
       const uint32_t* list = rp.preds.list + rp.preds.off[s];
-      for (uint32_t k0 = 0; k0 < npred && !fused; k0 += 32) {
-        const bool some = k0 + lane < npred;
-        fused = WaitSettled(m.mask, own, some ? list[k0 + lane] : own, some, r.stats, rp.wait_limit_ns);
+      for (uint32_t k0 = 0; k0 < npred && !fused; k0 += 128) {
+        uint32_t pixel[4], some = 0u;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const uint32_t k = k0 + 32u * i + lane;
+          pixel[i] = k < npred ? list[k] : own;
+          some |= k < npred ? 1u << i : 0u;
+        }
+        fused = WaitSettled(m.mask, own, pixel, some, r.stats, rp.wait_limit_ns);
       }
     } else {
       for (int k = 0; k < cnt && !fused; ++k) {
@@ -1057,8 +1244,8 @@ __global__ void __launch_bounds__(32 * kReplayWarps) ReplayKernel(FMaps m, FCons
         const uint32_t c1 = rp.preds.claim_off[g + 1];
         for (uint32_t q0 = rp.preds.claim_off[g]; q0 < c1 && !fused; q0 += 32) {
           const uint32_t cl = q0 + lane < c1 ? rp.preds.claim_list[q0 + lane] : s;
-          fused = WaitSettled(m.mask, own, cl < s ? SeedPixel(m, rp.im, cl) : own, cl < s, r.stats,
-                              rp.wait_limit_ns);
+          const uint32_t pixel[4] = {cl < s ? SeedPixel(m, rp.im, cl) : own, own, own, own};
+          fused = WaitSettled(m.mask, own, pixel, cl < s ? 1u : 0u, r.stats, rp.wait_limit_ns);
         }
       }
     }
@@ -1071,17 +1258,27 @@ __global__ void __launch_bounds__(32 * kReplayWarps) ReplayKernel(FMaps m, FCons
     if (rp.times) tw1 = GlobalTimer();
     // Masks are read from L2 (ld.global.cg): other SMs wrote them; a batch of
     // loads is in flight at once.
-    {
-      int k = lane;
-      for (; k + 96 < cnt; k += 128) {
-        const uint8_t a0 = __ldcg(m.mask + rgid[k]), a1 = __ldcg(m.mask + rgid[k + 32]),
-                      a2 = __ldcg(m.mask + rgid[k + 64]), a3 = __ldcg(m.mask + rgid[k + 96]);
-        flags[k] = a0;
-        flags[k + 32] = a1;
-        flags[k + 64] = a2;
-        flags[k + 96] = a3;
+    uint32_t open[4] = {0u, 0u, 0u, 0u};  // the same in every lane
+    if (in_regs) {
+      uint8_t f[4];
+#pragma unroll
+      for (int a = 0; a < 4; ++a) f[a] = lane + 32 * a < nopen ? __ldcg(m.mask + open_gid[a]) : 1;
+#pragma unroll
+      for (int a = 0; a < 4; ++a) {
+        open[a] = __ballot_sync(0xffffffffu, f[a] == 0);
+        if (lane + 32 * a < nopen) flags[sh.node[lane + 32 * a]] = f[a];
       }
-      for (; k < cnt; k += 32) flags[k] = __ldcg(m.mask + rgid[k]);
+    } else {
+      for (int k = lane; k < cnt; k += 128) {
+        const uint8_t a0 = __ldcg(m.mask + rgid[k]);
+        const uint8_t a1 = k + 32 < cnt ? __ldcg(m.mask + rgid[k + 32]) : 0;
+        const uint8_t a2 = k + 64 < cnt ? __ldcg(m.mask + rgid[k + 64]) : 0;
+        const uint8_t a3 = k + 96 < cnt ? __ldcg(m.mask + rgid[k + 96]) : 0;
+        flags[k] = a0;
+        if (k + 32 < cnt) flags[k + 32] = a1;
+        if (k + 64 < cnt) flags[k + 64] = a2;
+        if (k + 96 < cnt) flags[k + 96] = a3;
+      }
     }
     if (rp.level) {  // profiling: the longest chain of waits ending at this seed
       uint32_t lv = 0;
@@ -1104,52 +1301,35 @@ __global__ void __launch_bounds__(32 * kReplayWarps) ReplayKernel(FMaps m, FCons
     // max_traversal_depth) pixels are reachable (a pixel's traversal depth is
     // below the number fused); otherwise lane 0 replays the traversal itself.
     bool in_order = false;
-    if (node_sh) {
-      // Breadth-first search with the record's pixels as bits (fused before,
-      // or reached) and the reached pixels queued in acc: each wave expands
-      // only the frontier.
-      for (int k0 = 0; k0 < cnt; k0 += 32) {
-        const int k = k0 + lane;
-        const unsigned bal = __ballot_sync(0xffffffffu, k < cnt && flags[k] != 0);
-        if (lane == 0) sh.bits[k0 >> 5] = bal;
-      }
-      __syncwarp();
-      if (lane == 0) {
-        int t = 0;
-        if (!(sh.bits[0] & 1u)) {
-          sh.bits[0] |= 1u;
-          acc[0] = 0;
-          t = 1;
-        }
-        sh.qtail = t;
-      }
-      __syncwarp();
-      volatile int* vq = &sh.qtail;
-      volatile uint32_t* vb = sh.bits;
-      int qhead = 0, qt = *vq;
-      __syncwarp();
-      while (qhead < qt) {
-        for (int i = qhead + lane; i < qt; i += 32) {
-          const uint32_t k = acc[i];
-          for (uint32_t q = reoff[k], qe = reoff[k + 1]; q < qe; ++q) {
-            const uint32_t j = redges[q], bit = 1u << (j & 31u);
-            if (vb[j >> 5] & bit) continue;
-            if (!(atomicOr(&sh.bits[j >> 5], bit) & bit)) acc[atomicAdd(&sh.qtail, 1)] = (uint16_t)j;
+    if (in_regs) {
+      uint32_t seen[4] = {0u, 0u, 0u, 0u}, front[4] = {open[0] & 1u, 0u, 0u, 0u};
+      while (front[0] | front[1] | front[2] | front[3]) {
+        uint32_t next[4] = {0u, 0u, 0u, 0u};
+#pragma unroll
+        for (int a = 0; a < 4; ++a) {
+          seen[a] |= front[a];
+          if ((front[a] >> lane) & 1u) {
+#pragma unroll
+            for (int t = 0; t < 4; ++t) next[t] |= rows[a][t];
           }
         }
-        __syncwarp();
-        qhead = qt;
-        qt = *vq;
-        __syncwarp();
+#pragma unroll
+        for (int t = 0; t < 4; ++t) front[t] = __reduce_or_sync(0xffffffffu, next[t]) & open[t] & ~seen[t];
       }
-      int reach = qt;
+      int reach = 0;
+#pragma unroll
+      for (int a = 0; a < 4; ++a) {
+        if ((seen[a] >> lane) & 1u) acc[reach + __popc(seen[a] & ((1u << lane) - 1u))] = sh.node[lane + 32 * a];
+        reach += __popc(seen[a]);
+      }
+      __syncwarp();
       if (rp.times && lane == 0) {
         atomicAdd(rp.times + 3, (unsigned long long)cnt);
         atomicAdd(rp.times + 4, (unsigned long long)reach);
         if (reach > c.max_pix || reach > c.max_depth) atomicAdd(rp.times + 5, 1ull);
       }
       if (reach > c.max_pix || reach > c.max_depth) {  // flags still hold 1 = fused before
-        if (lane == 0) reach = SeqTraversal(flags, stack, acc, reoff, redges, c.max_pix, c.max_depth);
+        if (lane == 0) reach = traverse();
         reach = __shfl_sync(0xffffffffu, reach, 0);
         in_order = true;
       }
@@ -1165,7 +1345,7 @@ __global__ void __launch_bounds__(32 * kReplayWarps) ReplayKernel(FMaps m, FCons
           vf[k] = 3;
           any = true;
           for (uint32_t q = reoff[k], qe = reoff[k + 1]; q < qe; ++q) {
-            const uint32_t j = redges[q];
+            const uint32_t j = wide ? v.edges[q] : redges[q];
             if (vf[j] == 0) vf[j] = 2;
           }
         }
@@ -1188,7 +1368,7 @@ __global__ void __launch_bounds__(32 * kReplayWarps) ReplayKernel(FMaps m, FCons
       if (reach > c.max_pix || reach > c.max_depth) {
         for (int k = lane; k < cnt; k += 32) vf[k] = vf[k] == 1 ? 1 : 0;
         __syncwarp();
-        if (lane == 0) reach = SeqTraversal(flags, stack, acc, reoff, redges, c.max_pix, c.max_depth);
+        if (lane == 0) reach = traverse();
         reach = __shfl_sync(0xffffffffu, reach, 0);
         in_order = true;
       }
@@ -1218,44 +1398,88 @@ __global__ void __launch_bounds__(32 * kReplayWarps) ReplayKernel(FMaps m, FCons
     }
     // The fused point (:2098-2180).
     if (n < c.min_pix) continue;
-    // Images of the cluster, ascending.
-    for (int i = lane; i < n; i += 32) ids[i] = v.vid[acc[i]];
-    __syncwarp();
+    // Images of the cluster, ascending: as bits when there are at most 1024.
+    const bool few_views = m.num_views <= 1024;
     int nvis = 0;
-    for (int i0 = 0; i0 < n; i0 += 32) {
-      const int i = i0 + lane;
-      bool first = false;
-      if (i < n) {
-        first = true;
-        for (int j = 0; j < i; ++j)
-          if (ids[j] == ids[i]) {
-            first = false;
-            break;
-          }
+    if (few_views) {
+      sh.images[lane] = 0u;
+      __syncwarp();
+      for (int i = lane; i < n; i += 32) {
+        const uint32_t id = v.vid[acc[i]];
+        atomicOr(&sh.images[id >> 5], 1u << (id & 31u));
       }
-      nvis += __popc(__ballot_sync(0xffffffffu, first));
+      __syncwarp();
+      nvis = __reduce_add_sync(0xffffffffu, __popc(sh.images[lane]));
+    } else {
+      for (int i = lane; i < n; i += 32) ids[i] = v.vid[acc[i]];
+      __syncwarp();
+      for (int i0 = 0; i0 < n; i0 += 32) {
+        const int i = i0 + lane;
+        bool first = false;
+        if (i < n) {
+          first = true;
+          for (int j = 0; j < i; ++j)
+            if (ids[j] == ids[i]) {
+              first = false;
+              break;
+            }
+        }
+        nvis += __popc(__ballot_sync(0xffffffffu, first));
+      }
     }
     if (nvis < c.min_vis) continue;
     smvs_fused_point pt;
     memset(&pt, 0, sizeof(pt));
-    const float* maps[3] = {m.X, m.Y, m.Z};
+    const float* values = reinterpret_cast<const float*>(m.pix);  // 8 a pixel
+    // Up to 64 pixels: lane l keeps the values of pixels l and l + 32 of the
+    // cluster, all read at once, and the medians take them from there.
+    const bool small = n <= 64;
+    float4 e0a, e0b, e1a, e1b;
+    uint32_t c0 = 0, c1 = 0;
+    if (small) {
+      const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+      e0a = e0b = e1a = e1b = zero;
+      if (lane < n) {
+        const size_t g = rgid[acc[lane]];
+        e0a = m.pix[2 * g];
+        e0b = m.pix[2 * g + 1];
+        c0 = (uint32_t)m.rgb[3 * g] | (uint32_t)m.rgb[3 * g + 1] << 8 | (uint32_t)m.rgb[3 * g + 2] << 16;
+      }
+      if (lane + 32 < n) {
+        const size_t g = rgid[acc[lane + 32]];
+        e1a = m.pix[2 * g];
+        e1b = m.pix[2 * g + 1];
+        c1 = (uint32_t)m.rgb[3 * g] | (uint32_t)m.rgb[3 * g + 1] << 8 | (uint32_t)m.rgb[3 * g + 2] << 16;
+      }
+    }
     float xyz[3];
+#pragma unroll
     for (int a = 0; a < 3; ++a) {
-      for (int i = lane; i < n; i += 32) vals[i] = maps[a][rgid[acc[i]]];
-      __syncwarp();
-      xyz[a] = WarpMedian(vals, n, sh.med, lane);
+      if (small) {
+        xyz[a] = WarpMedian64(a == 0 ? e0a.x : a == 1 ? e0a.y : e0a.z, a == 0 ? e1a.x : a == 1 ? e1a.y : e1a.z, n,
+                              sh.vals, sh.med, lane);
+      } else {
+        for (int i = lane; i < n; i += 32) vals[i] = values[8 * (size_t)rgid[acc[i]] + a];
+        __syncwarp();
+        xyz[a] = WarpMedian(vals, n, sh.med, lane);
+      }
     }
     if (!isfinite(xyz[0]) || !isfinite(xyz[1]) || !isfinite(xyz[2])) continue;
     pt.x = xyz[0];
     pt.y = xyz[1];
     pt.z = xyz[2];
     if (c.with_normal) {
-      const float* nmaps[3] = {m.NX, m.NY, m.NZ};
       float fn[3];
+#pragma unroll
       for (int a = 0; a < 3; ++a) {
-        for (int i = lane; i < n; i += 32) vals[i] = nmaps[a][rgid[acc[i]]];
-        __syncwarp();
-        fn[a] = WarpMedian(vals, n, sh.med, lane);
+        if (small) {
+          fn[a] = WarpMedian64(a == 0 ? e0b.x : a == 1 ? e0b.y : e0b.z, a == 0 ? e1b.x : a == 1 ? e1b.y : e1b.z, n,
+                               sh.vals, sh.med, lane);
+        } else {
+          for (int i = lane; i < n; i += 32) vals[i] = values[8 * (size_t)rgid[acc[i]] + 4 + a];
+          __syncwarp();
+          fn[a] = WarpMedian(vals, n, sh.med, lane);
+        }
       }
       const float norm =
           __fsqrt_rn(__fadd_rn(__fadd_rn(__fmul_rn(fn[0], fn[0]), __fmul_rn(fn[1], fn[1])), __fmul_rn(fn[2], fn[2])));
@@ -1265,10 +1489,18 @@ __global__ void __launch_bounds__(32 * kReplayWarps) ReplayKernel(FMaps m, FCons
       pt.nz = __fdiv_rn(fn[2], norm);
     }
     uint8_t rgb[3];
+#pragma unroll
     for (int ch = 0; ch < 3; ++ch) {
-      for (int i = lane; i < n; i += 32) vals[i] = (float)m.rgb[3ull * rgid[acc[i]] + ch];
-      __syncwarp();
-      float med = roundf(WarpMedian(vals, n, sh.med, lane));
+      float med;
+      if (small) {
+        med = WarpMedian64((float)((c0 >> (8 * ch)) & 0xffu), (float)((c1 >> (8 * ch)) & 0xffu), n, sh.vals, sh.med,
+                           lane);
+      } else {
+        for (int i = lane; i < n; i += 32) vals[i] = (float)m.rgb[3ull * rgid[acc[i]] + ch];
+        __syncwarp();
+        med = WarpMedian(vals, n, sh.med, lane);
+      }
+      med = roundf(med);
       med = med < 255.0f ? med : 255.0f;  // TruncateCast<float, uint8_t>
       med = med > 0.0f ? med : 0.0f;
       rgb[ch] = (uint8_t)med;
@@ -1284,10 +1516,10 @@ __global__ void __launch_bounds__(32 * kReplayWarps) ReplayKernel(FMaps m, FCons
       if (!in_order) {
         for (int k = lane; k < cnt; k += 32) flags[k] = flags[k] == 1 ? 1 : 0;
         __syncwarp();
-        if (lane == 0) SeqTraversal(flags, stack, acc, reoff, redges, c.max_pix, c.max_depth);
+        if (lane == 0) traverse();
         __syncwarp();
       }
-      for (int i = lane; i < n; i += 32) vals[i] = m.G[rgid[acc[i]]];
+      for (int i = lane; i < n; i += 32) vals[i] = values[8 * (size_t)rgid[acc[i]] + 7];
       __syncwarp();
       if (lane == 0) {
         m_conf = 0.0f;
@@ -1298,9 +1530,15 @@ __global__ void __launch_bounds__(32 * kReplayWarps) ReplayKernel(FMaps m, FCons
     }
     m_conf = __fsub_rn(1.0f, m_conf);
     __syncwarp();
-    for (int i = lane + 1; i < n; i += 32) vals[i - 1] = v.derr[acc[i]];
-    __syncwarp();
-    const float med_err = WarpMedian(vals, n - 1, sh.med, lane);
+    float med_err;
+    if (n - 1 <= 64) {
+      med_err = WarpMedian64(lane + 1 < n ? v.derr[acc[lane + 1]] : 0.f, lane + 33 < n ? v.derr[acc[lane + 33]] : 0.f,
+                             n - 1, sh.vals, sh.med, lane);
+    } else {
+      for (int i = lane + 1; i < n; i += 32) vals[i - 1] = v.derr[acc[i]];
+      __syncwarp();
+      med_err = WarpMedian(vals, n - 1, sh.med, lane);
+    }
     float score = (float)((double)med_err / c.max_depth_error);
     const float mixed = __fadd_rn(__fmul_rn(0.6f, score), __fmul_rn(0.4f, m_conf));
     score = (1.0f < mixed) ? 1.0f : mixed;
@@ -1310,26 +1548,38 @@ __global__ void __launch_bounds__(32 * kReplayWarps) ReplayKernel(FMaps m, FCons
     uint32_t vbase = 0;
     if (lane == 0) vbase = (uint32_t)atomicAdd(rp.vis_cursor, (unsigned long long)nvis);
     vbase = __shfl_sync(0xffffffffu, vbase, 0);
-    for (int i = lane; i < n; i += 32) {
-      bool first = true;
-      for (int j = 0; j < i; ++j)
-        if (ids[j] == ids[i]) {
-          first = false;
-          break;
-        }
-      if (!first) continue;
-      int rank = 0;  // distinct images below this one
-      for (int j = 0; j < n; ++j) {
-        if (ids[j] >= ids[i]) continue;
-        bool fj = true;
-        for (int q = 0; q < j; ++q)
-          if (ids[q] == ids[j]) {
-            fj = false;
+    if (few_views) {
+      const uint32_t mine = sh.images[lane];
+      uint32_t before = (uint32_t)__popc(mine);
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, before, o);
+        if (lane >= o) before += y;
+      }
+      before -= (uint32_t)__popc(mine);
+      for (uint32_t left = mine; left; left &= left - 1u)
+        rp.vis_pool[vbase + before++] = (uint32_t)(32 * lane + __ffs((int)left) - 1);
+    } else {
+      for (int i = lane; i < n; i += 32) {
+        bool first = true;
+        for (int j = 0; j < i; ++j)
+          if (ids[j] == ids[i]) {
+            first = false;
             break;
           }
-        rank += fj ? 1 : 0;
+        if (!first) continue;
+        int rank = 0;  // distinct images below this one
+        for (int j = 0; j < n; ++j) {
+          if (ids[j] >= ids[i]) continue;
+          bool fj = true;
+          for (int q = 0; q < j; ++q)
+            if (ids[q] == ids[j]) {
+              fj = false;
+              break;
+            }
+          rank += fj ? 1 : 0;
+        }
+        rp.vis_pool[vbase + rank] = ids[i];
       }
-      rp.vis_pool[vbase + rank] = ids[i];
     }
     if (lane == 0) {
       rp.slot_pts[s] = pt;
@@ -1342,65 +1592,101 @@ __global__ void __launch_bounds__(32 * kReplayWarps) ReplayKernel(FMaps m, FCons
 }
 
 // ---- scan (exclusive, out[n] = total) ---------------------------------------
+// A block takes kScanItems items, a thread four uint4 of them; bound by memory
+// (with the four scans of an image in shared memory item by item: 0.13 ms more).
+__device__ __forceinline__ uint4 ScanLoad(const uint32_t* in, uint32_t i, uint32_t n) {
+  if (i + 4u <= n) return *reinterpret_cast<const uint4*>(in + i);  // i and the arrays are multiples of 4 words
+  uint4 x = make_uint4(0u, 0u, 0u, 0u);
+  if (i < n) x.x = in[i];
+  if (i + 1u < n) x.y = in[i + 1u];
+  if (i + 2u < n) x.z = in[i + 2u];
+  return x;
+}
+
 __global__ void __launch_bounds__(256) ScanReduceKernel(const uint32_t* in, uint32_t n, uint32_t* sums) {
-  __shared__ uint32_t red[256];
+  __shared__ uint32_t red[8];
   const uint32_t b0 = blockIdx.x * (uint32_t)kScanItems;
   uint32_t acc = 0;
-  for (int k = 0; k < kScanItems / 256; ++k) {
-    const uint32_t i = b0 + (uint32_t)k * 256u + threadIdx.x;
-    if (i < n) acc += in[i];
+#pragma unroll
+  for (int k = 0; k < kScanItems / 1024; ++k) {
+    const uint4 x = ScanLoad(in, b0 + (uint32_t)k * 1024u + 4u * threadIdx.x, n);
+    acc += x.x + x.y + x.z + x.w;
   }
-  red[threadIdx.x] = acc;
+  acc = __reduce_add_sync(0xffffffffu, acc);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
   __syncthreads();
-  for (int sft = 128; sft > 0; sft >>= 1) {
-    if ((int)threadIdx.x < sft) red[threadIdx.x] += red[threadIdx.x + sft];
-    __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < 8; ++w) acc += red[w];
+    sums[blockIdx.x] = acc;
   }
-  if (threadIdx.x == 0) sums[blockIdx.x] = red[0];
+}
+
+// Inclusive scan over the warp.
+__device__ __forceinline__ uint32_t WarpScan(uint32_t x, int lane) {
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+    if (lane >= o) x += y;
+  }
+  return x;
 }
 
 __global__ void __launch_bounds__(1024) ScanSumsKernel(uint32_t* sums, uint32_t nb) {
-  __shared__ uint32_t buf[1024];
+  __shared__ uint32_t part[32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   uint32_t carry = 0;
   for (uint32_t b0 = 0; b0 < nb; b0 += 1024) {
     const uint32_t i = b0 + threadIdx.x;
     const uint32_t x = i < nb ? sums[i] : 0u;
-    buf[threadIdx.x] = x;
+    const uint32_t incl = WarpScan(x, lane);
+    if (lane == 31) part[w] = incl;
     __syncthreads();
-    for (int sft = 1; sft < 1024; sft <<= 1) {
-      const uint32_t y = (int)threadIdx.x >= sft ? buf[threadIdx.x - sft] : 0u;
-      __syncthreads();
-      buf[threadIdx.x] += y;
-      __syncthreads();
-    }
-    if (i < nb) sums[i] = carry + buf[threadIdx.x] - x;
-    const uint32_t tot = buf[1023];
+    const uint32_t p = WarpScan(part[lane], lane);  // every warp: the warps' totals
+    const uint32_t before = w > 0 ? __shfl_sync(0xffffffffu, p, w - 1) : 0u;
+    const uint32_t total = __shfl_sync(0xffffffffu, p, 31);
+    if (i < nb) sums[i] = carry + before + incl - x;
+    carry += total;
     __syncthreads();
-    carry += tot;
   }
   if (threadIdx.x == 0) sums[nb] = carry;
 }
 
 __global__ void __launch_bounds__(256) ScanBlockKernel(const uint32_t* in, uint32_t n, const uint32_t* sums,
                                                        uint32_t nb, uint32_t* out) {
-  __shared__ uint32_t buf[256];
+  constexpr int kRounds = kScanItems / 1024;
+  __shared__ uint32_t part[kRounds][8];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const uint32_t b0 = blockIdx.x * (uint32_t)kScanItems;
+  uint4 x[kRounds];
+  uint32_t before[kRounds];  // items of the round before this thread's
+#pragma unroll
+  for (int k = 0; k < kRounds; ++k) {
+    x[k] = ScanLoad(in, b0 + (uint32_t)k * 1024u + 4u * threadIdx.x, n);
+    const uint32_t s = x[k].x + x[k].y + x[k].z + x[k].w;
+    const uint32_t incl = WarpScan(s, lane);
+    before[k] = incl - s;
+    if (lane == 31) part[k][w] = incl;
+  }
+  __syncthreads();
   uint32_t carry = sums[blockIdx.x];
-  for (int k = 0; k < kScanItems / 256; ++k) {
-    const uint32_t i = b0 + (uint32_t)k * 256u + threadIdx.x;
-    const uint32_t x = i < n ? in[i] : 0u;
-    buf[threadIdx.x] = x;
-    __syncthreads();
-    for (int sft = 1; sft < 256; sft <<= 1) {
-      const uint32_t y = (int)threadIdx.x >= sft ? buf[threadIdx.x - sft] : 0u;
-      __syncthreads();
-      buf[threadIdx.x] += y;
-      __syncthreads();
+#pragma unroll
+  for (int k = 0; k < kRounds; ++k) {
+    uint32_t at = carry + before[k];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const uint32_t t = part[k][j];
+      if (j < w) at += t;
+      carry += t;
     }
-    if (i < n) out[i] = carry + buf[threadIdx.x] - x;
-    const uint32_t tot = buf[255];
-    __syncthreads();
-    carry += tot;
+    const uint32_t i = b0 + (uint32_t)k * 1024u + 4u * threadIdx.x;
+    const uint4 o = make_uint4(at, at + x[k].x, at + x[k].x + x[k].y, at + x[k].x + x[k].y + x[k].z);
+    if (i + 4u <= n) {
+      *reinterpret_cast<uint4*>(out + i) = o;
+    } else {
+      if (i < n) out[i] = o.x;
+      if (i + 1u < n) out[i + 1u] = o.y;
+      if (i + 2u < n) out[i + 2u] = o.z;
+    }
   }
   if (blockIdx.x == nb - 1 && threadIdx.x == 0) out[n] = sums[nb];
 }
@@ -1460,8 +1746,9 @@ struct smvs_fusion {
   FView* d_views = nullptr;
   int* d_ov = nullptr;
   uint8_t* d_trav = nullptr;
-  float *d_D = nullptr, *d_X = nullptr, *d_Y = nullptr, *d_Z = nullptr, *d_NX = nullptr, *d_NY = nullptr,
-        *d_NZ = nullptr, *d_G = nullptr;
+  float4* d_pix = nullptr;    // 2 per pixel (FMaps::pix)
+  uint32_t* d_proj = nullptr; // FMaps::proj, when it fits
+  int deg = 0;                // overlapping images of the image that has most
   uint8_t* d_rgb = nullptr;
   uint8_t* d_mask = nullptr;
   uint32_t *d_claim_cnt = nullptr, *d_claim_off = nullptr, *d_claim_list = nullptr;
@@ -1571,8 +1858,7 @@ void FreeAll(smvs_fusion* f) {
   Harvest(f);
   if (f->pool) {
     Free(f, f->d_views); Free(f, f->d_ov); Free(f, f->d_trav);
-    Free(f, f->d_D); Free(f, f->d_X); Free(f, f->d_Y); Free(f, f->d_Z);
-    Free(f, f->d_NX); Free(f, f->d_NY); Free(f, f->d_NZ); Free(f, f->d_G);
+    Free(f, f->d_pix); Free(f, f->d_proj);
     Free(f, f->d_rgb); Free(f, f->d_mask);
     Free(f, f->d_claim_cnt); Free(f, f->d_claim_off); Free(f, f->d_claim_list);
     Free(f, f->d_pool); Free(f, f->d_rec_off); Free(f, f->d_over_list); Free(f, f->d_seq);
@@ -1669,14 +1955,10 @@ FMaps Maps(const smvs_fusion* f) {
   m.views = f->d_views;
   m.ov = f->d_ov;
   m.trav = f->d_trav;
-  m.D = f->d_D;
-  m.X = f->d_X;
-  m.Y = f->d_Y;
-  m.Z = f->d_Z;
-  m.NX = f->d_NX;
-  m.NY = f->d_NY;
-  m.NZ = f->d_NZ;
-  m.G = f->d_G;
+  m.pix = f->d_pix;
+  m.proj = f->d_proj;
+  m.deg = f->deg;
+  m.num_views = f->num_views;
   m.rgb = f->d_rgb;
   m.mask = f->d_mask;
   return m;
@@ -1786,8 +2068,8 @@ int FuseImage(smvs_fusion* f, int image) {
   ++f->launches;
   {
     ProfScope ps(f, SMVS_FUSION_KERNEL_CLOSURE);
-    ClosureKernel<<<f->closure_blocks, 32 * kClosureWarps, kClosureSmem, f->stream>>>(m, f->consts, im, Recs(f),
-                                                                                         0, f->d_stage);
+    (f->d_proj ? ClosureKernel<true> : ClosureKernel<false>)<<<f->closure_blocks, 32 * kClosureWarps, kClosureSmem,
+                                                              f->stream>>>(m, f->consts, im, Recs(f), 0, f->d_stage);
     ++f->launches;
   }
   FU_CUDA(cudaGetLastError());
@@ -1829,8 +2111,8 @@ int FuseImage(smvs_fusion* f, int image) {
     FU_CUDA(cudaMemcpyAsync(f->d_stats + 2, &status, sizeof(status), cudaMemcpyHostToDevice, f->stream));
     {
       ProfScope ps(f, SMVS_FUSION_KERNEL_CLOSURE);
-      ClosureKernel<<<f->closure_blocks, 32 * kClosureWarps, kClosureSmem, f->stream>>>(m, f->consts, im,
-                                                                                           Recs(f), 1, f->d_stage);
+      (f->d_proj ? ClosureKernel<true> : ClosureKernel<false>)<<<f->closure_blocks, 32 * kClosureWarps, kClosureSmem,
+                                                              f->stream>>>(m, f->consts, im, Recs(f), 1, f->d_stage);
       ++f->launches;
     }
     FU_CUDA(cudaGetLastError());
@@ -2226,8 +2508,7 @@ int smvs_fusion_create(const smvs_fusion_options* opt, const smvs_fusion_view* v
   const size_t T = (size_t)f->total;
   const size_t nov = std::max<size_t>((size_t)overlap_offsets[num_views], 1);
   if ((st = Alloc(f, &f->d_views, (size_t)num_views)) || (st = Alloc(f, &f->d_ov, nov)) ||
-      (st = Alloc(f, &f->d_trav, (size_t)num_views)) || (st = Alloc(f, &f->d_D, T)) || (st = Alloc(f, &f->d_X, T)) ||
-      (st = Alloc(f, &f->d_Y, T)) || (st = Alloc(f, &f->d_Z, T)) || (st = Alloc(f, &f->d_G, T)) ||
+      (st = Alloc(f, &f->d_trav, (size_t)num_views)) || (st = Alloc(f, &f->d_pix, 2 * T)) ||
       (st = Alloc(f, &f->d_rgb, 3 * T)) || (st = Alloc(f, &f->d_mask, T)) || (st = Alloc(f, &f->d_claim_cnt, T)) ||
       (st = Alloc(f, &f->d_claim_off, T + 1)) || (st = Alloc(f, &f->d_vis_pool, T)) ||
       (st = Alloc(f, &f->d_out_pts, T / 2 + 1)) || (st = Alloc(f, &f->d_out_visoff, T / 2 + 2)) ||
@@ -2235,9 +2516,6 @@ int smvs_fusion_create(const smvs_fusion_options* opt, const smvs_fusion_view* v
       (st = Alloc(f, &f->d_n_over, 1)) || (st = Alloc(f, &f->d_stats, 3)) || (st = Alloc(f, &f->d_used, 1)) ||
       (st = Alloc(f, &f->d_pred_used, 1)) ||
       (st = Alloc(f, &f->d_vis_cursor, 1)) || (st = Alloc(f, &f->d_totals, 2)))
-    return fail(st);
-  if (opt->with_normal &&
-      ((st = Alloc(f, &f->d_NX, T)) || (st = Alloc(f, &f->d_NY, T)) || (st = Alloc(f, &f->d_NZ, T))))
     return fail(st);
   // Record pool: 64 words per pixel of the largest image to start with; grows on demand.
   uint64_t max_px = 1;
@@ -2250,6 +2528,7 @@ int smvs_fusion_create(const smvs_fusion_options* opt, const smvs_fusion_view* v
   // device memory); it grows if an image needs more.
   int max_deg = 0;
   for (int v = 0; v < num_views; ++v) max_deg = std::max(max_deg, overlap_offsets[v + 1] - overlap_offsets[v]);
+  f->deg = max_deg;
   const double radius = std::max(opt->max_reproj_error, 0.5);
   const uint64_t disk = (uint64_t)std::ceil((2.0 * radius + 1.0) * (2.0 * radius + 1.0));
   const uint32_t cnt_est = (uint32_t)std::min<uint64_t>(kCap, disk * (uint64_t)(1 + max_deg));
@@ -2259,6 +2538,12 @@ int smvs_fusion_create(const smvs_fusion_options* opt, const smvs_fusion_view* v
   est = std::min<uint64_t>(est, std::max<uint64_t>(free_b / 16, max_px * 64ull));
   f->pool_words = (size_t)std::min<uint64_t>(std::max<uint64_t>(est, max_px * 64ull), 0xfffffff0ull);
   if ((st = Alloc(f, &f->d_pool, f->pool_words))) return fail(st);
+  // The projection table: a word per pixel and overlapping image (845 MB for 11
+  // views 1600x1200), when that is at most an eighth of the free memory; else the
+  // closures project in place.
+  if (max_deg > 0 && T * (size_t)max_deg * sizeof(uint32_t) <= free_b / 8 &&
+      (st = Alloc(f, &f->d_proj, T * (size_t)max_deg)))
+    return fail(st);
   auto up = [&](void* dst, const void* src, size_t bytes) -> cudaError_t {
     return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDefault, f->stream);
   };
@@ -2280,8 +2565,12 @@ int smvs_fusion_create(const smvs_fusion_options* opt, const smvs_fusion_view* v
     if (!f->used[v]) continue;
     const FView& hv = f->h_views[v];
     const size_t plane = (size_t)hv.W * hv.H;
-    if (cudaMemcpyAsync(f->d_D + hv.base, views[v].depth, plane * 4, kind, f->stream) != cudaSuccess)
-      return fail(Fail(SMVS_ECUDA, "fusion: depth map copy failed"));
+    float* d_depth = const_cast<float*>(views[v].depth);
+    if (memory == SMVS_MEM_HOST) {
+      if ((st = Alloc(f, &d_depth, plane))) return fail(st);
+      if (cudaMemcpyAsync(d_depth, views[v].depth, plane * 4, kind, f->stream) != cudaSuccess)
+        return fail(Fail(SMVS_ECUDA, "fusion: depth map copy failed"));
+    }
     if (views[v].color &&
         cudaMemcpyAsync(f->d_rgb + 3ull * hv.base, views[v].color, plane * 3, kind, f->stream) != cudaSuccess)
       return fail(Fail(SMVS_ECUDA, "fusion: color copy failed"));
@@ -2297,10 +2586,17 @@ int smvs_fusion_create(const smvs_fusion_options* opt, const smvs_fusion_view* v
     }
     const float* R = views[v].R;
     PointMapKernel<<<Blocks(plane, 256), 256, 0, f->stream>>>(
-        hv, R[0], R[1], R[2], R[3], R[4], R[5], R[6], R[7], R[8], d_normal, c.with_normal,
-        views[v].color != nullptr, f->d_D, f->d_X, f->d_Y, f->d_Z, f->d_NX, f->d_NY, f->d_NZ, f->d_G, f->d_rgb);
+        hv, R[0], R[1], R[2], R[3], R[4], R[5], R[6], R[7], R[8], d_depth, d_normal, c.with_normal,
+        views[v].color != nullptr, f->d_pix, f->d_rgb);
     ++f->launches;
-    if (memory == SMVS_MEM_HOST) Free(f, d_normal);
+    if (f->d_proj) {
+      ProjectTableKernel<<<Blocks(plane, 256), 256, 0, f->stream>>>(Maps(f), v, f->d_proj);
+      ++f->launches;
+    }
+    if (memory == SMVS_MEM_HOST) {
+      Free(f, d_depth);
+      Free(f, d_normal);
+    }
     if (cudaGetLastError() != cudaSuccess) return fail(Fail(SMVS_ECUDA, "fusion: point map launch failed"));
   }
   // The caller's maps are not referenced after this point.
@@ -2311,9 +2607,9 @@ int smvs_fusion_create(const smvs_fusion_options* opt, const smvs_fusion_view* v
       cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, f->device) != cudaSuccess || per_sm < 1)
     return fail(Fail(SMVS_ECUDA, "fusion: cannot size the replay grid"));
   f->replay_blocks = per_sm * sms;
-  if (cudaFuncSetAttribute(ClosureKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kClosureSmem) !=
-          cudaSuccess ||
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, ClosureKernel, 32 * kClosureWarps, kClosureSmem) !=
+  const auto closure = f->d_proj ? ClosureKernel<true> : ClosureKernel<false>;
+  if (cudaFuncSetAttribute(closure, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kClosureSmem) != cudaSuccess ||
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, closure, 32 * kClosureWarps, kClosureSmem) !=
           cudaSuccess ||
       per_sm < 1)
     return fail(Fail(SMVS_ECUDA, "fusion: cannot size the closure grid"));
