@@ -86,6 +86,10 @@ int smvs_test_calibrate(int kind, double seconds, double* rate);
  * pixels or replay_stack stack entries replay from global scratch instead of
  * shared memory. Results do not change; the paths taken do. */
 int smvs_test_fusion_caps(int closure_cap, int replay_cap, int replay_stack);
+/* Paths of fusions created from now on by this thread that large inputs take:
+ * in_place = 1: closures project in place (no projection table); walk = 1: the
+ * replay walks the claims of a record's pixels (no predecessor lists). */
+int smvs_test_fusion_paths(int in_place, int walk);
 
 /* With profiling on during smvs_fusion_run: per fused image (in fusion order)
  * the longest chain of seeds that each waited for the previous one (the

@@ -272,6 +272,7 @@ _SIGNATURES = {
                                            C.c_float, C.c_float, C.POINTER(C.c_double), C.POINTER(C.c_double), C.POINTER(C.c_double),
                                            C.c_int, C.c_int, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p]),
     "smvs_test_fusion_caps": (C.c_int, [C.c_int, C.c_int, C.c_int]),
+    "smvs_test_fusion_paths": (C.c_int, [C.c_int, C.c_int]),
     "smvs_test_fusion_chains": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_int, C.POINTER(C.c_int)]),
     "smvs_test_fusion_image_ms": (C.c_int, [C.c_void_p, C.c_void_p, C.c_int, C.POINTER(C.c_int)]),
     "smvs_test_fusion_replay_times": (C.c_int, [C.c_void_p, C.c_void_p, C.c_int, C.POINTER(C.c_int)]),

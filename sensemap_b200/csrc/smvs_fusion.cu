@@ -69,6 +69,9 @@ constexpr unsigned long long kWaitLimitNs = 20ull * 1000 * 1000 * 1000;  // boun
 // successors are never released, for this thread's next runs.
 thread_local unsigned long long t_wait_limit_ns = 0;  // 0: kWaitLimitNs
 thread_local long long t_withhold = -1;
+// Test hook (smvs_test_fusion_paths) for fusions created on this thread: no
+// projection table; no predecessor lists.
+thread_local bool t_in_place = false, t_walk = false;
 
 // Status bits written by the kernels.
 constexpr uint32_t kStTimeout = 1u, kStPool = 2u, kStBad = 4u, kStBig = 8u;
@@ -1749,6 +1752,7 @@ struct smvs_fusion {
   float4* d_pix = nullptr;    // 2 per pixel (FMaps::pix)
   uint32_t* d_proj = nullptr; // FMaps::proj, when it fits
   int deg = 0;                // overlapping images of the image that has most
+  bool walk = false;          // test hook: the replay walks the claims
   uint8_t* d_rgb = nullptr;
   uint8_t* d_mask = nullptr;
   uint32_t *d_claim_cnt = nullptr, *d_claim_off = nullptr, *d_claim_list = nullptr;
@@ -1982,7 +1986,7 @@ FPreds Preds(const smvs_fusion* f) {
   p.cnt = f->d_pred_cnt;
   p.list = f->d_pred_list;
   p.used = f->d_pred_used;
-  p.cap = std::min<unsigned long long>(f->claim_list_cap, 0xffffffffull);
+  p.cap = f->walk ? 0ull : std::min<unsigned long long>(f->claim_list_cap, 0xffffffffull);
   p.claim_off = f->d_claim_off;
   p.claim_list = f->d_claim_list;
   return p;
@@ -2541,7 +2545,8 @@ int smvs_fusion_create(const smvs_fusion_options* opt, const smvs_fusion_view* v
   // The projection table: a word per pixel and overlapping image (845 MB for 11
   // views 1600x1200), when that is at most an eighth of the free memory; else the
   // closures project in place.
-  if (max_deg > 0 && T * (size_t)max_deg * sizeof(uint32_t) <= free_b / 8 &&
+  f->walk = t_walk;
+  if (!t_in_place && max_deg > 0 && T * (size_t)max_deg * sizeof(uint32_t) <= free_b / 8 &&
       (st = Alloc(f, &f->d_proj, T * (size_t)max_deg)))
     return fail(st);
   auto up = [&](void* dst, const void* src, size_t bytes) -> cudaError_t {
@@ -2767,6 +2772,12 @@ int smvs_test_fusion_replay_times(smvs_fusion* f, double* out, int capacity, int
     o[7] = (double)ti[7] / seeds / 1000.0;
     o[8] = (double)ti[8] / seeds / 1000.0;
   }
+  return SMVS_OK;
+}
+
+int smvs_test_fusion_paths(int in_place, int walk) {
+  t_in_place = in_place != 0;
+  t_walk = walk != 0;
   return SMVS_OK;
 }
 
