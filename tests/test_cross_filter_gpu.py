@@ -205,3 +205,34 @@ def test_cross_filter_pool_reuse_and_release():
     c = _gpu_run(opt, views, problems)
     for k in range(len(views)):
         assert np.array_equal(a["vis"][k], c["vis"][k])
+
+
+@pytest.mark.parametrize("max_cost,thr", [(0.0, 0.01), (1e-3, 0.05), (0.7, 0.02), (3e19, 3.0)])
+def test_cross_filter_edges_bit_exact(max_cost, thr):
+    """Problems of different sizes in one launch (listed blocks) and of equal ones
+    (computed blocks), pixels whose depth is NaN, infinite, huge, tiny or negative, and
+    the bound on the squared distance at 0, an inexact square and past the largest float."""
+    from oracle.oracle import FilterView
+    from sensemap_b200 import synthetic as syn
+    scene = syn.planes_scene(seed=11, width=131, height=75, focal=110.0, num_src=6)
+    rng = np.random.default_rng(5)
+    odd = np.array([np.nan, np.inf, -np.inf, 3e38, 1e-30, -2.0, 0.0], np.float32)
+    for sizes in ({}, {1: (67, 131), 4: (75, 33)}):
+        views = []
+        for k, (v, (d, n)) in enumerate(zip(scene.views, syn.noisy_maps(scene, seed=2))):
+            h, w = sizes.get(k, d.shape)
+            d, n = d[:h, :w].copy(), n[:, :h, :w].copy()
+            hit = rng.random(d.shape) < 0.02
+            d[hit] = rng.choice(odd, int(hit.sum()))
+            views.append(FilterView(v.K, v.R, v.T, d, n, ref_flag=True))
+        problems = [(r, [s for s in range(len(views)) if s != r]) for r in range(len(views))]
+        opt = PatchMatchOptions(filter_geom_consistency_max_cost=max_cost, depth_diff_threshold=thr,
+                                filter_min_num_consistent=2)
+        got = _gpu_run(opt, views, problems)
+        refined, vis, delta, dd = _oracle(opt, views, problems)
+        for r in refined:
+            np.testing.assert_array_equal(got["refined"][r], refined[r])  # NaN where NaN
+            np.testing.assert_array_equal(got["delta"][r], delta[r])
+        for k in range(len(views)):
+            np.testing.assert_array_equal(got["vis"][k], vis[k])
+            np.testing.assert_array_equal(got["dedup"][k], dd[k])
