@@ -39,6 +39,46 @@ def test_resample_maps_match_oracle(shape, new):
     np.testing.assert_array_equal(on.cpu().numpy(), orc.resample_maps(n, *new, True))
 
 
+@pytest.mark.parametrize("shape,new", [((1003, 1001), (499, 501)), ((1002, 998), (501, 499)), ((700, 720), (701, 731)),
+                                       ((611, 1640), (30, 820))])
+def test_rescale_image_of_many_outputs_a_thread(shape, new):
+    """Four outputs a thread (the row pass has at least half a million), with rows and
+    columns left over and taps at the borders, on both sides of the line."""
+    import torch
+    rng = np.random.default_rng(7)
+    img = np.round(rng.uniform(0, 255, shape)).astype(np.float32)
+    assert shape[0] * new[1] >= 498000
+    out, _ = rescale_image(torch.from_numpy(img).cuda(), new[1], new[0])
+    torch.cuda.synchronize()
+    np.testing.assert_array_equal(out.cpu().numpy(), orc.rescale_image(img, *new))
+
+
+@pytest.mark.parametrize("shape,new", [((33, 41), (67, 40)), ((7, 5), (150, 33)), ((1, 1), (9, 3)), ((40, 31), (41, 93)),
+                                       ((90, 70), (23, 140)), ((5, 64), (3, 64))])
+@pytest.mark.parametrize("which", ["depth", "normal", "both"])
+def test_resample_maps_one_or_both(shape, new, which):
+    """Several output rows a thread (the map grows) and one (it does not), each map alone
+    and both in one launch, ratios that share input rows unevenly."""
+    import torch
+
+    from sensemap_b200 import _native as N
+    rng = np.random.default_rng(8)
+    d = rng.uniform(-1, 10, shape).astype(np.float32)
+    n = rng.normal(0, 1, (3,) + shape).astype(np.float32)
+    n[:, rng.random(shape) < 0.2] = 0
+    td, tn = torch.from_numpy(d).cuda(), torch.from_numpy(n).cuda()
+    od = torch.full(new, -7.0, device="cuda")
+    on = torch.full((3,) + new, -7.0, device="cuda")
+    with_d, with_n = which != "normal", which != "depth"
+    N.check(N.lib().smvs_resample_maps(td.data_ptr() if with_d else None, tn.data_ptr() if with_n else None, shape[1],
+                                       shape[0], od.data_ptr(), on.data_ptr(), new[1], new[0], None))
+    torch.cuda.synchronize()
+    want_d = orc.resample_maps(d[None], *new, False)[0] if with_d else np.full(new, -7.0, np.float32)
+    want_n = orc.resample_maps(n, *new, True) if with_n else np.full((3,) + new, -7.0, np.float32)
+    np.testing.assert_array_equal(od.cpu().numpy(), want_d)
+    np.testing.assert_array_equal(on.cpu().numpy(), want_n)
+
+
 def test_level_sizes():
     assert level_size(6000, 4000, 0)[:2] == (6000, 4000)
     assert level_size(6000, 4000, 1)[:2] == (3000, 2000)
