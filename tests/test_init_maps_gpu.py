@@ -109,3 +109,38 @@ def test_heightfield_mesh_larger(scene):
         _same(IM.init_depth_from_mesh(W, H, v.K, v.R, v.T, X, F, FN), ref)
         m = (ref[0] > 0) & (v.depth_gt > 0)
         assert np.median(np.abs(ref[0][m] - v.depth_gt[m]) / v.depth_gt[m]) < 0.01
+
+
+@pytest.mark.parametrize("w,h", [(1, 9), (64, 2), (33, 47), (301, 203)])
+@pytest.mark.parametrize("count", [1, 31, 700, 30000])
+def test_point_windows_bit_exact(w, h, count):
+    """Windows of each size the scatter has a form for, over the borders, with few and
+    many points a group of lanes, ties, culled and NaN points."""
+    rng = np.random.default_rng(count + w)
+    K = np.array([[40.0, 0, w / 2], [0, 40.0, h / 2], [0, 0, 1]])
+    R, T = np.eye(3), np.zeros(3)
+    z = rng.choice([1.0, 1.5, 2.0, 2.0000001], count)
+    u, v = rng.uniform(-2, w + 1, count), rng.uniform(-2, h + 1, count)
+    pts = np.stack([(u - w / 2) / 40 * z, (v - h / 2) / 40 * z, z], 1).astype(np.float32)
+    nrm = rng.normal(0, 1, (count, 3)).astype(np.float32)
+    nrm[:, 2] = -np.abs(nrm[:, 2])
+    pts[rng.random(count) < 0.02] = np.nan
+    pts[rng.random(count) < 0.02, 2] *= -1
+    for level in range(5):
+        _same(IM.init_depth_from_dense_points(w, h, K, R, T, pts, nrm, level=level),
+              O.init_from_dense_points(w, h, K, R, T, pts, nrm, level))
+    _same(IM.init_depth_from_sparse_points(w, h, K, R, T, pts), O.init_from_sparse_points(w, h, K, R, T, pts))
+
+
+@pytest.mark.parametrize("step", [3, 8, 41, 90])
+def test_mesh_of_small_and_large_faces(scene, step):
+    """Boxes on both sides of the size from which a warp walks them, in any mixture."""
+    v = scene.views[0]
+    H, W = v.depth_gt.shape
+    parts = [syn.grid_mesh(scene, 0, step=s, duplicate_frac=0.3, seed=s) for s in (step, 6)]
+    X = np.concatenate([parts[0][0], parts[1][0]])
+    F = np.concatenate([parts[0][1], parts[1][1] + len(parts[0][0])]).astype(np.int32)
+    FN = np.concatenate([parts[0][2], parts[1][2]])
+    order = np.random.default_rng(step).permutation(len(F))
+    F, FN = F[order], FN[order]
+    _same(IM.init_depth_from_mesh(W, H, v.K, v.R, v.T, X, F, FN), O.init_from_mesh(W, H, v.K, v.R, v.T, X, F, FN))
