@@ -2242,76 +2242,317 @@ int CheckStatus(smvs_fusion* f) {
 }
 
 // ---- clean-up passes after the image loop ----------------------------------
-// The fused cloud on the host (points, visibility offsets, image indices).
-struct HostCloud {
-  std::vector<smvs_fused_point> pts;
-  std::vector<uint64_t> off;
-  std::vector<uint32_t> vis;
+// The passes work on the cloud where it lies. Their scratch is what the image loop
+// has left: the pixel records (32 bytes a pixel), the claims and the visibility
+// pool are not read after it, and Run may be called once.
+struct Carve {
+  smvs_fusion* f;
+  char* at;
+  size_t left;
+  void* own[8] = {};
+  int nown = 0;
+  explicit Carve(smvs_fusion* fusion)
+      : f(fusion), at(reinterpret_cast<char*>(fusion->d_pix)), left(32 * (size_t)fusion->total) {}
+  ~Carve() {
+    for (int k = 0; k < nown; ++k) cudaFreeAsync(own[k], f->stream);
+  }
+  template <typename T>
+  int Take(T** p, size_t count) {
+    const size_t bytes = (std::max<size_t>(count * sizeof(T), 1) + 255) / 256 * 256;
+    if (bytes <= left) {
+      *p = reinterpret_cast<T*>(at);
+      at += bytes;
+      left -= bytes;
+      return SMVS_OK;
+    }
+    if (nown == (int)(sizeof(own) / sizeof(own[0]))) return Fail(SMVS_ENOMEM, "fusion: too many scratch arrays");
+    const int st = Alloc(f, p, count);
+    if (!st) own[nown++] = *p;
+    return st;
+  }
 };
 
-int Download(smvs_fusion* f, HostCloud& c) {
-  c.pts.resize(f->num_points);
-  c.off.resize(f->num_points + 1);
-  c.vis.resize(f->num_vis);
-  if (f->num_points)
-    FU_CUDA(cudaMemcpyAsync(c.pts.data(), f->d_out_pts, f->num_points * sizeof(smvs_fused_point),
-                            cudaMemcpyDeviceToHost, f->stream));
-  FU_CUDA(cudaMemcpyAsync(c.off.data(), f->d_out_visoff, (f->num_points + 1) * sizeof(uint64_t),
-                          cudaMemcpyDeviceToHost, f->stream));
-  if (f->num_vis)
-    FU_CUDA(cudaMemcpyAsync(c.vis.data(), f->d_out_vis, f->num_vis * sizeof(uint32_t), cudaMemcpyDeviceToHost,
-                            f->stream));
-  FU_CUDA(cudaStreamSynchronize(f->stream));
-  return SMVS_OK;
+// Per point: its number of images where it is kept, else 0.
+__global__ void KeptCountKernel(uint32_t n, const uint64_t* __restrict__ off, const uint32_t* __restrict__ keep,
+                                uint32_t* __restrict__ nvis) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) nvis[i] = keep[i] ? (uint32_t)(off[i + 1] - off[i]) : 0u;
 }
 
-// Keeps the points with keep[i] (order preserved, as the reference's in-place
-// compaction loops do) and writes the cloud back to the device arrays, which
-// only shrink.
-int CompactUpload(smvs_fusion* f, HostCloud& c, const std::vector<uint8_t>& keep, size_t* removed) {
-  size_t j = 0, v = 0;
-  for (size_t i = 0; i < c.pts.size(); ++i) {
-    if (!keep[i]) continue;
-    const uint64_t b = c.off[i], e = c.off[i + 1];
-    c.pts[j] = c.pts[i];
-    c.off[j] = v;
-    for (uint64_t k = b; k < e; ++k) c.vis[v++] = c.vis[k];
-    ++j;
+__global__ void KeepKernel(uint32_t n, const uint32_t* __restrict__ keep, const uint32_t* __restrict__ pt_idx,
+                           const uint32_t* __restrict__ vis_idx, const smvs_fused_point* __restrict__ pts,
+                           const uint64_t* __restrict__ off, const uint32_t* __restrict__ vis,
+                           smvs_fused_point* __restrict__ new_pts, uint64_t* __restrict__ new_off,
+                           uint32_t* __restrict__ new_vis) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i > n) return;
+  const uint32_t j = pt_idx[i], v = vis_idx[i];
+  if (i == n) {
+    new_off[j] = v;
+    return;
   }
-  c.off[j] = v;
-  if (removed) *removed = c.pts.size() - j;
-  if (j) FU_CUDA(cudaMemcpyAsync(f->d_out_pts, c.pts.data(), j * sizeof(smvs_fused_point), cudaMemcpyHostToDevice,
-                                 f->stream));
-  FU_CUDA(cudaMemcpyAsync(f->d_out_visoff, c.off.data(), (j + 1) * sizeof(uint64_t), cudaMemcpyHostToDevice,
-                          f->stream));
-  if (v) FU_CUDA(cudaMemcpyAsync(f->d_out_vis, c.vis.data(), v * sizeof(uint32_t), cudaMemcpyHostToDevice, f->stream));
+  if (!keep[i]) return;
+  new_pts[j] = pts[i];
+  new_off[j] = v;
+  const uint64_t b = off[i];
+  const uint32_t cnt = (uint32_t)(off[i + 1] - b);
+  for (uint32_t k = 0; k < cnt; ++k) new_vis[v + k] = vis[b + k];
+}
+
+// Keeps the points with keep[i] (1 or 0; order preserved, as the reference's
+// in-place compaction loops do). The device arrays stay where they are and only shrink.
+int Compact(smvs_fusion* f, Carve& scratch, const uint32_t* keep, size_t* removed) {
+  const uint32_t n = (uint32_t)f->num_points;
+  uint32_t *nvis, *pt_idx, *vis_idx, *new_vis = f->d_claim_cnt;
+  smvs_fused_point* new_pts;
+  uint64_t* new_off;
+  int st;
+  if ((st = scratch.Take(&nvis, n)) || (st = scratch.Take(&pt_idx, (size_t)n + 1)) ||
+      (st = scratch.Take(&vis_idx, (size_t)n + 1)) || (st = scratch.Take(&new_pts, n)) ||
+      (st = scratch.Take(&new_off, (size_t)n + 1)))
+    return st;
+  const int blocks = Blocks((size_t)n + 1, 256);
+  KeptCountKernel<<<blocks, 256, 0, f->stream>>>(n, f->d_out_visoff, keep, nvis);
+  if ((st = Scan(f, keep, n, pt_idx)) || (st = Scan(f, nvis, n, vis_idx))) return st;
+  KeepKernel<<<blocks, 256, 0, f->stream>>>(n, keep, pt_idx, vis_idx, f->d_out_pts, f->d_out_visoff, f->d_out_vis,
+                                            new_pts, new_off, new_vis);
+  f->launches += 2;
+  FU_CUDA(cudaGetLastError());
+  uint32_t j = 0, v = 0;
+  FU_CUDA(cudaMemcpyAsync(&j, pt_idx + n, 4, cudaMemcpyDeviceToHost, f->stream));
+  FU_CUDA(cudaMemcpyAsync(&v, vis_idx + n, 4, cudaMemcpyDeviceToHost, f->stream));
   FU_CUDA(cudaStreamSynchronize(f->stream));
+  if (j) FU_CUDA(cudaMemcpyAsync(f->d_out_pts, new_pts, j * sizeof(smvs_fused_point), cudaMemcpyDeviceToDevice,
+                                 f->stream));
+  FU_CUDA(cudaMemcpyAsync(f->d_out_visoff, new_off, ((size_t)j + 1) * 8, cudaMemcpyDeviceToDevice, f->stream));
+  if (v) FU_CUDA(cudaMemcpyAsync(f->d_out_vis, new_vis, (size_t)v * 4, cudaMemcpyDeviceToDevice, f->stream));
+  FU_CUDA(cudaStreamSynchronize(f->stream));
+  if (removed) *removed = n - j;
   f->num_points = j;
   f->num_vis = v;
   return SMVS_OK;
 }
 
-// Eigen 3.3's float evaluation of K * (R * X + T) (coefficient-based 3x3
-// products reduce as (p0 + p1) + p2), then proj / z rounded half away from
-// zero (std::round), as RemoveDuplicatePoints projects (fusion.cc:2216-2219).
-void ProjectPoint(const smvs_fusion_view& v, const smvs_fused_point& p, int* u, int* w) {
-  const float X[3] = {p.x, p.y, p.z};
-  float c[3], q[3];
-  for (int r = 0; r < 3; ++r) c[r] = ((v.R[3 * r] * X[0] + v.R[3 * r + 1] * X[1]) + v.R[3 * r + 2] * X[2]) + v.T[r];
-  for (int r = 0; r < 3; ++r) q[r] = (v.K[3 * r] * c[0] + v.K[3 * r + 1] * c[1]) + v.K[3 * r + 2] * c[2];
-  *u = (int)std::round(q[0] / q[2]);
-  *w = (int)std::round(q[1] / q[2]);
+// RemoveDuplicatePoints (fusion.cc:2184-2266): points in fusion order claim the
+// pixel they project to in each of their images; a point meeting an occupant seen
+// by more images is dropped (and looks no further), otherwise it takes the pixel
+// and the occupant is dropped. The occupants of a pixel are seen by ever more (or as
+// many) images, so point i is stopped at a pixel exactly if an earlier point seen by
+// more images took it, and is dropped there exactly if a later point took it too.
+// Points of one number of images do not stop one another: from the largest number
+// down, each level is two launches over its points (where is each stopped; the
+// pixels before that are taken), then one over all points finds the dropped ones. A
+// walk on the host took 7 ms for 66,000 points of 6 views 640x480 (and the cloud's
+// way there and back), now 0.2 ms; 470,000 of 11 views 1600x1200 110 ms, now 0.5 ms.
+struct DupView {
+  float K[9], R[9], T[3];
+  int W, H;
+  uint32_t base;
+};
+constexpr uint32_t kNoCell = 0xffffffffu;
+constexpr int kDupBins = 1024;  // numbers of images counted in shared memory
+
+__global__ void __launch_bounds__(256) DupLevelsKernel(uint32_t n, const uint64_t* __restrict__ off, int max_level,
+                                                       uint32_t* __restrict__ counts) {
+  __shared__ uint32_t bins[kDupBins];
+  for (int k = threadIdx.x; k < kDupBins; k += 256) bins[k] = 0;
+  __syncthreads();
+  for (uint32_t i = blockIdx.x * 256 + threadIdx.x; i < n; i += gridDim.x * 256) {
+    const int level = (int)min(off[i + 1] - off[i], (uint64_t)max_level);
+    atomicAdd(level < kDupBins ? bins + level : counts + level, 1u);
+  }
+  __syncthreads();
+  for (int k = threadIdx.x; k < min(kDupBins, max_level + 1); k += 256)
+    if (bins[k]) atomicAdd(counts + k, bins[k]);
 }
 
-// Exact k-nearest-neighbour spacing on a uniform grid. Points are bucketed by
-// cell (counting sort); each query scans cubes of growing half-width r cells
-// around its own cell, keeping the K smallest squared distances (double, the
-// coordinate differences squared and summed x, y, z as CGAL's Euclidean
-// distance does), and stops once K are known and the K-th lies within r cell
-// widths (every point nearer than that is inside the scanned cube; a 1e-9
-// relative margin covers the rounding of the cell assignment) or the cube
-// covers the grid.
+// Lists the points by level: cursor[level] starts at the level's first place.
+__global__ void DupOrderKernel(uint32_t n, const uint64_t* __restrict__ off, int max_level,
+                               uint32_t* __restrict__ cursor, uint32_t* __restrict__ list) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const int level = (int)min(off[i + 1] - off[i], (uint64_t)max_level);
+  const unsigned same = __match_any_sync(__activemask(), level);
+  const int lane = threadIdx.x % 32, leader = __ffs(same) - 1;
+  uint32_t first = 0;
+  if (lane == leader) first = atomicAdd(cursor + level, (uint32_t)__popc(same));
+  first = __shfl_sync(same, first, leader);
+  list[first + __popc(same & ((1u << lane) - 1))] = i;
+}
+
+// Eigen 3.3's float evaluation of K * (R * X + T) (coefficient-based 3x3 products
+// reduce as (p0 + p1) + p2), then proj / z rounded half away from zero (std::round),
+// as RemoveDuplicatePoints projects (fusion.cc:2216-2219); kNoCell outside the image
+// and where an int cannot hold the result.
+__device__ __forceinline__ uint32_t DupCell(const DupView& v, const smvs_fused_point& p) {
+  float c[3], q[3];
+  for (int r = 0; r < 3; ++r) c[r] = ((v.R[3 * r] * p.x + v.R[3 * r + 1] * p.y) + v.R[3 * r + 2] * p.z) + v.T[r];
+  for (int r = 0; r < 3; ++r) q[r] = (v.K[3 * r] * c[0] + v.K[3 * r + 1] * c[1]) + v.K[3 * r + 2] * c[2];
+  const float u = roundf(q[0] / q[2]), w = roundf(q[1] / q[2]);
+  if (!(u >= 0.0f && u < (float)v.W && w >= 0.0f && w < (float)v.H)) return kNoCell;
+  const int iu = (int)u, iw = (int)w;
+  if (iu >= v.W || iw >= v.H) return kNoCell;  // sizes that a float rounds up
+  return v.base + (uint32_t)iw * (uint32_t)v.W + (uint32_t)iu;
+}
+
+// earliest[cell]: the first point of a higher level that took the cell.
+__global__ void DupStopKernel(const uint32_t* __restrict__ list, uint32_t count,
+                              const smvs_fused_point* __restrict__ pts, const uint64_t* __restrict__ off,
+                              const uint32_t* __restrict__ vis, const DupView* __restrict__ views,
+                              const uint32_t* __restrict__ earliest, uint32_t* __restrict__ cells,
+                              uint32_t* __restrict__ keep) {
+  const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= count) return;
+  const uint32_t i = list[t];
+  const smvs_fused_point p = pts[i];
+  bool stopped = false;
+  for (uint64_t k = off[i]; k < off[i + 1]; ++k) {
+    uint32_t cell = stopped ? kNoCell : DupCell(views[vis[k]], p);
+    if (cell != kNoCell && earliest[cell] < i) {
+      stopped = true;
+      cell = kNoCell;
+    }
+    cells[k] = cell;
+  }
+  keep[i] = !stopped;
+}
+
+__global__ void DupTakeKernel(const uint32_t* __restrict__ list, uint32_t count, const uint64_t* __restrict__ off,
+                              const uint32_t* __restrict__ cells, uint32_t* __restrict__ earliest,
+                              uint32_t* __restrict__ latest) {
+  const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= count) return;
+  const uint32_t i = list[t];
+  for (uint64_t k = off[i]; k < off[i + 1]; ++k) {
+    const uint32_t cell = cells[k];
+    if (cell == kNoCell) continue;
+    atomicMin(earliest + cell, i);
+    atomicMax(latest + cell, i);
+  }
+}
+
+__global__ void DupDropKernel(uint32_t n, const uint64_t* __restrict__ off, const uint32_t* __restrict__ cells,
+                              const uint32_t* __restrict__ latest, uint32_t* __restrict__ keep) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  bool dropped = false;
+  for (uint64_t k = off[i]; k < off[i + 1] && !dropped; ++k) dropped = cells[k] != kNoCell && latest[cells[k]] > i;
+  if (dropped) keep[i] = 0;
+}
+
+// ---- outliers ---------------------------------------------------------------
+// Order-preserving map float -> uint32, for minima and maxima.
+__host__ __device__ __forceinline__ uint32_t FloatKey(float f) {
+  uint32_t b;
+  memcpy(&b, &f, 4);
+  return (b & 0x80000000u) ? ~b : (b | 0x80000000u);
+}
+__host__ __device__ __forceinline__ float KeyFloat(uint32_t k) {
+  const uint32_t b = (k & 0x80000000u) ? (k & 0x7fffffffu) : ~k;
+  float f;
+  memcpy(&f, &b, 4);
+  return f;
+}
+
+// The numbers that the outlier pass gathers over the cloud: keys of the smallest
+// (even) and largest (odd) x, y, z and score, and the score histogram. A NaN takes
+// no part in a minimum or maximum (std::min and std::max with it second).
+struct CloudStats {
+  uint32_t range[8];
+  uint32_t bins[256];
+};
+
+__global__ void StatsResetKernel(CloudStats* __restrict__ s) {
+  const int t = threadIdx.x;
+  if (t < 8) s->range[t] = t & 1 ? 0u : 0xffffffffu;
+  s->bins[t] = 0;
+}
+
+__device__ __forceinline__ void FoldKeys(const uint32_t (&key)[8], int first, int last, CloudStats* s) {
+  for (int k = first; k < last; ++k) {
+    const uint32_t v = k & 1 ? __reduce_max_sync(0xffffffffu, key[k]) : __reduce_min_sync(0xffffffffu, key[k]);
+    if (threadIdx.x % 32 != 0) continue;
+    if (k & 1) atomicMax(s->range + k, v);
+    else atomicMin(s->range + k, v);
+  }
+}
+
+__global__ void __launch_bounds__(256) CloudBoxKernel(const smvs_fused_point* __restrict__ pts, uint32_t n,
+                                                      CloudStats* __restrict__ s) {
+  uint32_t key[8] = {0xffffffffu, 0u, 0xffffffffu, 0u, 0xffffffffu, 0u, 0xffffffffu, 0u};
+  for (uint32_t i = blockIdx.x * 256 + threadIdx.x; i < n; i += gridDim.x * 256) {
+    const float x[3] = {pts[i].x, pts[i].y, pts[i].z};
+    for (int a = 0; a < 3; ++a)
+      if (!isnan(x[a])) {
+        key[2 * a] = min(key[2 * a], FloatKey(x[a]));
+        key[2 * a + 1] = max(key[2 * a + 1], FloatKey(x[a]));
+      }
+  }
+  FoldKeys(key, 0, 6, s);
+}
+
+// Blends each score with its spacing ratio (fusion.cc:2542-2611) and finds the range.
+__global__ void __launch_bounds__(256) ScoreKernel(smvs_fused_point* __restrict__ pts, uint32_t n,
+                                                   const float* __restrict__ spacing, int blend, double unit,
+                                                   CloudStats* __restrict__ s) {
+  uint32_t key[8] = {0xffffffffu, 0u, 0xffffffffu, 0u, 0xffffffffu, 0u, 0xffffffffu, 0u};
+  for (uint32_t i = blockIdx.x * 256 + threadIdx.x; i < n; i += gridDim.x * 256) {
+    float score = pts[i].score;
+    if (blend) {
+      const float factor = (float)((double)spacing[i] / unit);
+      score = (float)((double)score * 0.6 + (double)factor * 0.4);
+      pts[i].score = score;
+    }
+    if (!isnan(score)) {
+      key[6] = min(key[6], FloatKey(score));
+      key[7] = max(key[7], FloatKey(score));
+    }
+  }
+  FoldKeys(key, 6, 8, s);
+}
+
+// One score for every point (range 0) puts all points in bin 0: none is dropped
+// (the reference divides 0 by 0 there).
+__device__ __forceinline__ int ScoreBin(float score, float smin, float range) {
+  if (!(range > 0)) return 0;
+  const float gray = (score - smin) / range;
+  return min(max((int)(gray * 255), 0), 255);
+}
+
+__global__ void __launch_bounds__(256) HistKernel(const smvs_fused_point* __restrict__ pts, uint32_t n,
+                                                  CloudStats* __restrict__ s) {
+  __shared__ uint32_t bins[256];
+  bins[threadIdx.x] = 0;
+  __syncthreads();
+  const float smin = KeyFloat(s->range[6]), range = KeyFloat(s->range[7]) - smin;
+  for (uint32_t i = blockIdx.x * 256 + threadIdx.x; i < n; i += gridDim.x * 256)
+    atomicAdd(bins + ScoreBin(pts[i].score, smin, range), 1u);
+  __syncthreads();
+  if (bins[threadIdx.x]) atomicAdd(s->bins + threadIdx.x, bins[threadIdx.x]);
+}
+
+struct BinMask {
+  uint32_t drop[8];  // a bit per bin
+};
+
+__global__ void BinKeepKernel(const smvs_fused_point* __restrict__ pts, uint32_t n, const CloudStats* __restrict__ s,
+                              BinMask mask, uint32_t* __restrict__ keep) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const float smin = KeyFloat(s->range[6]), range = KeyFloat(s->range[7]) - smin;
+  const int b = ScoreBin(pts[i].score, smin, range);
+  keep[i] = !((mask.drop[b / 32] >> (b % 32)) & 1u);
+}
+
+// Exact k-nearest-neighbour spacing on a uniform grid. Points are bucketed by cell
+// (counting sort, positions copied into cell order); a query scans the cube of
+// half-width r cells around its own cell, keeping the K smallest squared distances
+// (double, the coordinate differences squared and summed x, y, z as CGAL's Euclidean
+// distance does), and doubles r until the K-th lies within r cell widths (every
+// point nearer than that is inside the cube) or the cube covers the grid. A margin
+// of 1e-7 covers the rounding of the cell assignment.
 constexpr int kMaxKnn = 64;
+constexpr double kKnnMargin = 1.0 - 1e-7;
 
 struct KnnGrid {
   double minx, miny, minz, h, inv_h;
@@ -2335,66 +2576,111 @@ __global__ void KnnCountKernel(const smvs_fused_point* __restrict__ pts, uint32_
   atomicAdd(counts + cell, 1u);
 }
 
-__global__ void KnnScatterKernel(uint32_t n, const uint32_t* __restrict__ cell_of, const uint32_t* __restrict__ start,
-                                 uint32_t* __restrict__ cursor, uint32_t* __restrict__ sorted) {
+// sorted: position and (in w) index of the points, by cell; uses the counts up.
+__global__ void KnnScatterKernel(const smvs_fused_point* __restrict__ pts, uint32_t n,
+                                 const uint32_t* __restrict__ cell_of, const uint32_t* __restrict__ start,
+                                 uint32_t* __restrict__ counts, float4* __restrict__ sorted) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const uint32_t c = cell_of[i];
-  sorted[start[c] + atomicAdd(cursor + c, 1u)] = i;
+  sorted[start[c] + atomicSub(counts + c, 1u) - 1u] = make_float4(pts[i].x, pts[i].y, pts[i].z, __uint_as_float(i));
 }
+
+// The kReg smallest distances met, in order.
+template <int kReg>
+struct Nearest {
+  double best[kReg];
+  __device__ __forceinline__ void Reset() {
+#pragma unroll
+    for (int k = 0; k < kReg; ++k) best[k] = INFINITY;
+  }
+  __device__ __forceinline__ void Add(double d, int K) {
+    if constexpr (kReg <= 16) {  // in registers
+      if (!(d < best[kReg - 1])) return;
+#pragma unroll
+      for (int k = kReg - 1; k > 0; --k) best[k] = d < best[k - 1] ? best[k - 1] : (d < best[k] ? d : best[k]);
+      best[0] = d < best[0] ? d : best[0];
+    } else {
+      if (!(d < best[K - 1])) return;
+      int m = K - 1;
+      while (m > 0 && best[m - 1] > d) { best[m] = best[m - 1]; --m; }
+      best[m] = d;
+    }
+  }
+  __device__ __forceinline__ double At(int j) const {
+    if constexpr (kReg <= 16) {
+      double v = best[0];
+#pragma unroll
+      for (int k = 1; k < kReg; ++k) v = k == j ? best[k] : v;
+      return v;
+    } else {
+      return best[j];
+    }
+  }
+};
 
 // ComputeAverageDistance's per-point spacing (patch_match_controller.cc:160-181):
 // the mean distance of the query's K = nb_neighbors + 1 nearest points (itself
 // included, at distance 0) over K - 1, accumulated nearest first in float with
-// each distance added in double.
-__global__ void KnnSpacingKernel(const smvs_fused_point* __restrict__ pts, uint32_t n, KnnGrid g,
-                                 const uint32_t* __restrict__ start, const uint32_t* __restrict__ sorted, int K,
-                                 float* __restrict__ spacing) {
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const double qx = pts[i].x, qy = pts[i].y, qz = pts[i].z;
+// each distance added in double. Queries go in cell order, so a warp reads the same
+// cells; a cube's cells of one row (along x) are one range of `sorted`; rows that
+// lie further than the K-th distance are passed over. Up to 16 distances stay in
+// registers. 65,000 points, K = 7: the whole pass takes 0.48 ms (0.69 ms
+// with a cell per point), with queries in point order, cells read one by one and the
+// points through an index 1.65 ms; 470,000 points 1.34 ms (1 cell a point 2.19, 27
+// 1.12). On the host's side of it the cloud went both ways: 3.95 and 24.2 ms.
+template <int kReg>
+__global__ void __launch_bounds__(128) KnnSpacingKernel(const float4* __restrict__ sorted, uint32_t n, KnnGrid g,
+                                                        const uint32_t* __restrict__ start, int K,
+                                                        float* __restrict__ spacing) {
+  const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= n) return;
+  const float4 q = __ldg(sorted + t);
+  const uint32_t i = __float_as_uint(q.w);
+  const double qx = q.x, qy = q.y, qz = q.z;
+  if (isnan(q.x) || isnan(q.y) || isnan(q.z)) {
+    spacing[i] = NAN;
+    return;
+  }
   const int cx = CellCoord(qx, g.minx, g.inv_h, g.gx);
   const int cy = CellCoord(qy, g.miny, g.inv_h, g.gy);
   const int cz = CellCoord(qz, g.minz, g.inv_h, g.gz);
-  double best[kMaxKnn];
-  int cnt = 0;
-  const int rmax = max(g.gx, max(g.gy, g.gz));
-  for (int r = 0; r <= rmax; ++r) {
-    // Cells at Chebyshev distance exactly r from the query's cell.
-    for (int z = cz - r; z <= cz + r; ++z) {
-      if (z < 0 || z >= g.gz) continue;
-      for (int y = cy - r; y <= cy + r; ++y) {
-        if (y < 0 || y >= g.gy) continue;
-        // Inner rows of the shell hold only its two end cells.
-        const bool face = (z == cz - r || z == cz + r || y == cy - r || y == cy + r);
-        const int step = face ? 1 : 2 * r;
-        for (int x = cx - r; x <= cx + r; x += step) {
-          if (x < 0 || x >= g.gx) continue;
-          const uint32_t cell = ((uint32_t)z * g.gy + (uint32_t)y) * g.gx + (uint32_t)x;
-          for (uint32_t k = start[cell]; k < start[cell + 1]; ++k) {
-            const smvs_fused_point& p = pts[sorted[k]];
-            const double dx = qx - (double)p.x, dy = qy - (double)p.y, dz = qz - (double)p.z;
-            double d = dx * dx;
-            d += dy * dy;
-            d += dz * dz;
-            if (cnt < K) {
-              int m = cnt++;
-              while (m > 0 && best[m - 1] > d) { best[m] = best[m - 1]; --m; }
-              best[m] = d;
-            } else if (d < best[K - 1]) {
-              int m = K - 1;
-              while (m > 0 && best[m - 1] > d) { best[m] = best[m - 1]; --m; }
-              best[m] = d;
-            }
-          }
+  Nearest<kReg> near;
+  for (int r = 1;; r = r < (1 << 28) ? 2 * r : r) {
+    near.Reset();
+    const int x0 = max(cx - r, 0), x1 = min(cx + r, g.gx - 1), y0 = max(cy - r, 0), y1 = min(cy + r, g.gy - 1),
+              z0 = max(cz - r, 0), z1 = min(cz + r, g.gz - 1);
+    double kth = INFINITY;
+    for (int z = z0; z <= z1; ++z) {
+      const double dz = (double)max(abs(z - cz) - 1, 0) * (g.h * kKnnMargin);
+      if (dz * dz > kth) continue;
+      for (int y = y0; y <= y1; ++y) {
+        const double dy = (double)max(abs(y - cy) - 1, 0) * (g.h * kKnnMargin);
+        if (dz * dz + dy * dy > kth) continue;
+        const uint32_t row = ((uint32_t)z * g.gy + (uint32_t)y) * g.gx;
+        const uint32_t end = __ldg(start + row + x1 + 1);
+        for (uint32_t k = __ldg(start + row + x0); k < end; ++k) {
+          const float4 p = __ldg(sorted + k);
+          const double dx = qx - (double)p.x, ey = qy - (double)p.y, ez = qz - (double)p.z;
+          double d = dx * dx;
+          d += ey * ey;
+          d += ez * ez;
+          near.Add(d, K);
         }
+        kth = near.At(K - 1);
       }
     }
-    const double reach = (double)r * g.h * (1.0 - 1e-9);
-    if (cnt == K && best[K - 1] <= reach * reach) break;
+    const double reach = (double)r * (g.h * kKnnMargin);
+    if (kth <= reach * reach || (x1 - x0 + 1 == g.gx && y1 - y0 + 1 == g.gy && z1 - z0 + 1 == g.gz)) break;
   }
   float s = 0.0f;
-  for (int k = 0; k < cnt; ++k) s = (float)((double)s + sqrt(best[k]));
+  int cnt = 0;
+  for (int k = 0; k < K; ++k) {
+    const double d = near.At(k);
+    if (d == INFINITY) break;
+    s = (float)((double)s + sqrt(d));
+    ++cnt;
+  }
   if (cnt > 1) s /= (float)(cnt - 1);
   spacing[i] = s;
 }
@@ -2801,46 +3087,58 @@ int smvs_fusion_remove_duplicate_points(smvs_fusion* f, size_t* num_removed) {
   if (!f) return Fail(SMVS_EINVAL, "null fusion");
   if (!f->ran) return Fail(SMVS_ESTATE, "fusion: run first");
   if (cudaSetDevice(f->device) != cudaSuccess) return Fail(SMVS_ECUDA, "fusion: cannot use GPU %d", f->device);
-  HostCloud c;
-  int st = Download(f, c);
-  if (st) return st;
-  // RemoveDuplicatePoints (fusion.cc:2184-2266): points in fusion order claim
-  // the pixel they project to in each of their images; a point meeting an
-  // occupant seen by more images is dropped (and looks no further), otherwise
-  // it takes the pixel and the occupant is dropped.
-  // Occupants as int32 like the reference's Mat<int> (fewer than 2^31 points:
-  // the views hold fewer than 2^31 pixels).
-  std::vector<std::vector<int32_t>> occ(f->num_views);
-  for (int v = 0; v < f->num_views; ++v)
-    occ[v].assign((size_t)f->views[v].width * (size_t)f->views[v].height, -1);
-  const size_t n = c.pts.size();
-  std::vector<uint8_t> removal(n, 0);
-  for (size_t i = 0; i < n; ++i) {
-    if (removal[i]) continue;
-    const uint64_t nvis = c.off[i + 1] - c.off[i];
-    for (uint64_t k = c.off[i]; k < c.off[i + 1]; ++k) {
-      const int img = (int)c.vis[k];
-      const smvs_fusion_view& v = f->views[img];
-      int u, w;
-      ProjectPoint(v, c.pts[i], &u, &w);
-      if (u < 0 || u >= v.width || w < 0 || w >= v.height) continue;
-      int32_t& o = occ[img][(size_t)w * v.width + u];
-      if (o == -1) {
-        o = (int32_t)i;
-        continue;
-      }
-      const uint64_t ovis = c.off[o + 1] - c.off[o];
-      if (ovis > nvis) {
-        removal[i] = 1;
-        break;
-      }
-      removal[o] = 1;
-      o = (int32_t)i;
-    }
+  if (num_removed) *num_removed = 0;
+  const uint32_t n = (uint32_t)f->num_points;  // at most half the pixels, fewer than 2^30
+  if (n == 0) return SMVS_OK;
+  const int max_level = f->num_views;  // a point lists an image once
+  uint32_t *cells = f->d_vis_pool, *earliest = f->d_claim_cnt, *latest = f->d_claim_off;
+  uint32_t *keep, *list, *counts;
+  DupView* d_views;
+  Carve scratch(f);
+  int st;
+  if ((st = scratch.Take(&keep, n)) || (st = scratch.Take(&list, n)) ||
+      (st = scratch.Take(&counts, (size_t)max_level + 1)) || (st = scratch.Take(&d_views, (size_t)f->num_views)))
+    return st;
+  std::vector<DupView> views(f->num_views);
+  for (int v = 0; v < f->num_views; ++v) {
+    const smvs_fusion_view& fv = f->views[v];
+    memcpy(views[v].K, fv.K, sizeof(fv.K));
+    memcpy(views[v].R, fv.R, sizeof(fv.R));
+    memcpy(views[v].T, fv.T, sizeof(fv.T));
+    views[v].W = f->h_views[v].W;
+    views[v].H = f->h_views[v].H;
+    views[v].base = f->h_views[v].base;
   }
-  std::vector<uint8_t> keep(n);
-  for (size_t i = 0; i < n; ++i) keep[i] = !removal[i];
-  return CompactUpload(f, c, keep, num_removed);
+  FU_CUDA(cudaMemcpyAsync(d_views, views.data(), views.size() * sizeof(DupView), cudaMemcpyHostToDevice, f->stream));
+  FU_CUDA(cudaMemsetAsync(counts, 0, ((size_t)max_level + 1) * 4, f->stream));
+  FU_CUDA(cudaMemsetAsync(earliest, 0xff, (size_t)f->total * 4, f->stream));
+  FU_CUDA(cudaMemsetAsync(latest, 0, (size_t)f->total * 4, f->stream));
+  DupLevelsKernel<<<std::min<uint32_t>(Blocks(n, 256), 296), 256, 0, f->stream>>>(n, f->d_out_visoff, max_level, counts);
+  FU_CUDA(cudaGetLastError());
+  std::vector<uint32_t> count((size_t)max_level + 1), start((size_t)max_level + 1);
+  FU_CUDA(cudaMemcpyAsync(count.data(), counts, count.size() * 4, cudaMemcpyDeviceToHost, f->stream));
+  FU_CUDA(cudaStreamSynchronize(f->stream));
+  uint32_t at = 0;
+  for (int level = max_level; level >= 0; --level) {
+    start[level] = at;
+    at += count[level];
+  }
+  FU_CUDA(cudaMemcpyAsync(counts, start.data(), start.size() * 4, cudaMemcpyHostToDevice, f->stream));
+  DupOrderKernel<<<Blocks(n, 256), 256, 0, f->stream>>>(n, f->d_out_visoff, max_level, counts, list);
+  f->launches += 2;
+  for (int level = max_level; level >= 0; --level) {
+    if (!count[level]) continue;
+    DupStopKernel<<<Blocks(count[level], 128), 128, 0, f->stream>>>(list + start[level], count[level], f->d_out_pts,
+                                                                    f->d_out_visoff, f->d_out_vis, d_views, earliest,
+                                                                    cells, keep);
+    DupTakeKernel<<<Blocks(count[level], 128), 128, 0, f->stream>>>(list + start[level], count[level], f->d_out_visoff,
+                                                                    cells, earliest, latest);
+    f->launches += 2;
+  }
+  DupDropKernel<<<Blocks(n, 256), 256, 0, f->stream>>>(n, f->d_out_visoff, cells, latest, keep);
+  ++f->launches;
+  FU_CUDA(cudaGetLastError());
+  return Compact(f, scratch, keep, num_removed);
 }
 
 int smvs_fusion_remove_outliers(smvs_fusion* f, int nb_neighbors, double max_spacing_factor, size_t* num_removed) {
@@ -2854,15 +3152,30 @@ int smvs_fusion_remove_outliers(smvs_fusion* f, int nb_neighbors, double max_spa
   const size_t n = f->num_points;
   if (n == 0) return SMVS_OK;
   if (n >= (1ull << 32) - 1) return Fail(SMVS_EINVAL, "fusion: too many points for the neighbour grid");
-  HostCloud c;
-  int st = Download(f, c);
-  if (st) return st;
-  // Grid: about one cell per point over the bounding box (cells of equal
-  // side, at least one per axis, at most 2^24 per axis).
-  double lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
-  for (const auto& p : c.pts) {
-    const double x[3] = {p.x, p.y, p.z};
-    for (int a = 0; a < 3; ++a) { lo[a] = std::min(lo[a], x[a]); hi[a] = std::max(hi[a], x[a]); }
+  const uint32_t nn = (uint32_t)n;
+  Carve scratch(f);
+  CloudStats* stats;
+  uint32_t* keep;
+  int st;
+  if ((st = scratch.Take(&stats, 1)) || (st = scratch.Take(&keep, n))) return st;
+  const int sweep = std::min<uint32_t>(Blocks(n, 256), 296);
+  StatsResetKernel<<<1, 256, 0, f->stream>>>(stats);
+  CloudBoxKernel<<<sweep, 256, 0, f->stream>>>(f->d_out_pts, nn, stats);
+  f->launches += 2;
+  FU_CUDA(cudaGetLastError());
+  CloudStats h_stats;
+  FU_CUDA(cudaMemcpyAsync(h_stats.range, stats->range, sizeof(h_stats.range), cudaMemcpyDeviceToHost, f->stream));
+  FU_CUDA(cudaStreamSynchronize(f->stream));
+  // Grid over the bounding box: cells of equal side, at least one per axis, at most
+  // 2^24 per axis, about kCells per point. The points lie on surfaces, so an
+  // occupied cell holds about (n / kCells^2)^(1/3) of them (10 of 65,000) and a
+  // cube of 27 cells is near the smallest that holds the neighbours.
+  constexpr int kCells = 8;
+  double lo[3], hi[3];
+  for (int a = 0; a < 3; ++a) {
+    const bool any = h_stats.range[2 * a] <= h_stats.range[2 * a + 1];
+    lo[a] = any ? KeyFloat(h_stats.range[2 * a]) : INFINITY;
+    hi[a] = any ? KeyFloat(h_stats.range[2 * a + 1]) : -INFINITY;
   }
   if (!(std::isfinite(lo[0]) && std::isfinite(lo[1]) && std::isfinite(lo[2]) && std::isfinite(hi[0]) &&
         std::isfinite(hi[1]) && std::isfinite(hi[2])))
@@ -2875,53 +3188,39 @@ int smvs_fusion_remove_outliers(smvs_fusion* f, int nb_neighbors, double max_spa
     if (ext[a] > emax * 1e-6) vol *= ext[a];
     else ++flat;
   }
-  double h = emax > 0 ? std::pow(vol / (double)n, 1.0 / (3 - std::min(flat, 2))) : 1.0;
+  double h = emax > 0 ? std::pow(vol / ((double)kCells * (double)n), 1.0 / (3 - std::min(flat, 2))) : 1.0;
   if (!(h > 0)) h = 1.0;
   KnnGrid g;
   g.minx = lo[0]; g.miny = lo[1]; g.minz = lo[2];
   int dims[3];
   for (;;) {
     for (int a = 0; a < 3; ++a) dims[a] = (int)std::min(16777216.0, std::floor(ext[a] / h) + 1.0);
-    if ((double)dims[0] * dims[1] * dims[2] <= 4.0 * (double)n + 64.0) break;
+    if ((double)dims[0] * dims[1] * dims[2] <= std::min(2.0 * kCells * (double)n + 64.0, 2147483648.0)) break;
     h *= 1.26;
   }
   g.h = h; g.inv_h = 1.0 / h;
   g.gx = dims[0]; g.gy = dims[1]; g.gz = dims[2];
   const size_t cells = (size_t)g.gx * g.gy * g.gz;
-  uint32_t *cell_of = nullptr, *counts = nullptr, *startv = nullptr, *cursor = nullptr, *sorted = nullptr;
-  float* spacing = nullptr;
-  auto release = [&] {
-    Free(f, cell_of); Free(f, counts); Free(f, startv); Free(f, cursor); Free(f, sorted); Free(f, spacing);
-  };
-  if ((st = Alloc(f, &cell_of, n)) || (st = Alloc(f, &counts, cells)) || (st = Alloc(f, &startv, cells + 1)) ||
-      (st = Alloc(f, &cursor, cells)) || (st = Alloc(f, &sorted, n)) || (st = Alloc(f, &spacing, n))) {
-    release();
+  uint32_t *cell_of, *counts, *startv;
+  float4* sorted;
+  float* spacing;
+  if ((st = scratch.Take(&cell_of, n)) || (st = scratch.Take(&counts, cells)) ||
+      (st = scratch.Take(&startv, cells + 1)) || (st = scratch.Take(&sorted, n)) || (st = scratch.Take(&spacing, n)))
     return st;
-  }
-  const uint32_t nn = (uint32_t)n;
   const int K = nb_neighbors + 1;
-  if (cudaMemsetAsync(counts, 0, cells * sizeof(uint32_t), f->stream) != cudaSuccess ||
-      cudaMemsetAsync(cursor, 0, cells * sizeof(uint32_t), f->stream) != cudaSuccess) {
-    release();
-    return Fail(SMVS_ECUDA, "fusion: clearing the neighbour grid failed");
-  }
-  KnnCountKernel<<<(nn + 255) / 256, 256, 0, f->stream>>>(f->d_out_pts, nn, g, cell_of, counts);
-  st = Scan(f, counts, cells, startv);
-  if (!st) {
-    KnnScatterKernel<<<(nn + 255) / 256, 256, 0, f->stream>>>(nn, cell_of, startv, cursor, sorted);
-    KnnSpacingKernel<<<(nn + 127) / 128, 128, 0, f->stream>>>(f->d_out_pts, nn, g, startv, sorted, K, spacing);
-    f->launches += 3;
-  }
+  FU_CUDA(cudaMemsetAsync(counts, 0, cells * sizeof(uint32_t), f->stream));
+  KnnCountKernel<<<Blocks(n, 256), 256, 0, f->stream>>>(f->d_out_pts, nn, g, cell_of, counts);
+  if ((st = Scan(f, counts, cells, startv))) return st;
+  KnnScatterKernel<<<Blocks(n, 256), 256, 0, f->stream>>>(f->d_out_pts, nn, cell_of, startv, counts, sorted);
+  auto knn = K <= 8 ? KnnSpacingKernel<8> : K <= 16 ? KnnSpacingKernel<16> : KnnSpacingKernel<kMaxKnn>;
+  knn<<<Blocks(n, 128), 128, 0, f->stream>>>(sorted, nn, g, startv, K, spacing);
+  f->launches += 3;
+  FU_CUDA(cudaGetLastError());
   std::vector<float> dists(n);
-  if (!st && (cudaGetLastError() != cudaSuccess ||
-              cudaMemcpyAsync(dists.data(), spacing, n * sizeof(float), cudaMemcpyDeviceToHost, f->stream) !=
-                  cudaSuccess ||
-              cudaStreamSynchronize(f->stream) != cudaSuccess))
-    st = Fail(SMVS_ECUDA, "fusion: neighbour spacing kernels failed");
-  release();
-  if (st) return st;
+  FU_CUDA(cudaMemcpyAsync(dists.data(), spacing, n * sizeof(float), cudaMemcpyDeviceToHost, f->stream));
+  FU_CUDA(cudaStreamSynchronize(f->stream));
   // ComputeAverageDistance's mean (patch_match_controller.cc:184-227): a float
-  // sum in point order.
+  // sum in point order, whose roundings no other order gives.
   float average = 0.0f;
   for (size_t i = 0; i < n; ++i) average += dists[i];
   average /= (float)n;
@@ -2929,33 +3228,25 @@ int smvs_fusion_remove_outliers(smvs_fusion* f, int nb_neighbors, double max_spa
   // ratio, histogram the scores over 256 bins of [min, max], and drop points
   // in a bin holding under 1 % of the points at or above the 90th cumulative
   // percent.
-  if (average > 1e-6) {
-    for (size_t i = 0; i < n; ++i) {
-      const float factor = (float)((double)dists[i] / (max_spacing_factor * (double)average));
-      c.pts[i].score = (float)((double)c.pts[i].score * 0.6 + (double)factor * 0.4);
-    }
-  }
-  float smin = c.pts[0].score, smax = c.pts[0].score;
-  for (const auto& p : c.pts) { smin = std::min(smin, p.score); smax = std::max(smax, p.score); }
-  const float range = smax - smin;
-  // One score for every point (range 0) puts all points in bin 0: none is
-  // dropped (the reference divides 0 by 0 there).
-  auto bin = [&](float score) -> int {
-    if (!(range > 0)) return 0;
-    const float gray = (score - smin) / range;
-    return (int)(gray * 255);
-  };
-  std::vector<float> ratios(256, 0.0f), acc(256, 0.0f);
-  for (const auto& p : c.pts) ratios[bin(p.score)]++;
-  for (int k = 0; k < 256; ++k) ratios[k] /= (float)n;
+  ScoreKernel<<<sweep, 256, 0, f->stream>>>(f->d_out_pts, nn, spacing, average > 1e-6,
+                                            max_spacing_factor * (double)average, stats);
+  HistKernel<<<sweep, 256, 0, f->stream>>>(f->d_out_pts, nn, stats);
+  f->launches += 2;
+  FU_CUDA(cudaGetLastError());
+  FU_CUDA(cudaMemcpyAsync(h_stats.bins, stats->bins, sizeof(h_stats.bins), cudaMemcpyDeviceToHost, f->stream));
+  FU_CUDA(cudaStreamSynchronize(f->stream));
+  BinMask mask{};
   float sum = 0.0f;
-  for (int k = 0; k < 256; ++k) { sum += ratios[k]; acc[k] = sum; }
-  std::vector<uint8_t> keep(n);
-  for (size_t i = 0; i < n; ++i) {
-    const int b = bin(c.pts[i].score);
-    keep[i] = !((double)ratios[b] < 0.01 && (double)acc[b] >= 0.9);
+  for (int k = 0; k < 256; ++k) {
+    // The reference counts in floats, which stop at 2^24.
+    const float ratio = (float)std::min<uint32_t>(h_stats.bins[k], 1u << 24) / (float)n;
+    sum += ratio;
+    if ((double)ratio < 0.01 && (double)sum >= 0.9) mask.drop[k / 32] |= 1u << (k % 32);
   }
-  return CompactUpload(f, c, keep, num_removed);
+  BinKeepKernel<<<Blocks(n, 256), 256, 0, f->stream>>>(f->d_out_pts, nn, stats, mask, keep);
+  ++f->launches;
+  FU_CUDA(cudaGetLastError());
+  return Compact(f, scratch, keep, num_removed);
 }
 
 void smvs_fusion_destroy(smvs_fusion* f) {

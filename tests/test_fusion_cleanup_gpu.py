@@ -65,3 +65,40 @@ def test_outlier_pass_with_far_points_and_other_neighbour_counts():
         rp, ro, rv, o_removed, _ = O.fusion_remove_outliers(*before, nb_neighbors=nb, max_spacing_factor=3.0)
         assert removed == o_removed
         _same_cloud(after, (rp, ro, rv))
+
+
+@pytest.mark.parametrize("nb", [1, 7, 8, 15, 16, 63])
+def test_cleanup_of_scattered_points(nb):
+    """Loose fusion of noisy maps: points that stand alone (their neighbours lie many
+    cells away), every number of images, and each form of the neighbour search at the
+    ends of its range. The passes come in both orders and twice."""
+    scene = syn.heightfield_scene(seed=6, width=96, height=72, focal=72.0, num_src=5)
+    ims, ov = syn.fusion_inputs(scene, seed=4)
+    rng = np.random.default_rng(nb)
+    for im in ims:
+        hit = rng.random(im.depth.shape) < 0.1
+        im.depth[hit] *= rng.choice([0.3, 0.7, 1.6, 5.0], int(hit.sum())).astype(np.float32)
+    opt = FusionOptions(min_num_pixels=2, min_num_visible_images=2, max_normal_error=60.0, max_depth_error=0.05)
+    with StereoFusion(opt, ims, ov) as f:
+        f.Run()
+        cloud = _cloud(f)
+        assert len(cloud[0]) > 200
+        for k in range(4):
+            if k % 2 == 0:
+                removed = f.RemoveOutliers(nb_neighbors=nb, max_spacing_factor=2.0)
+                p, o, v, want, _ = O.fusion_remove_outliers(*cloud, nb_neighbors=nb, max_spacing_factor=2.0)
+            else:
+                removed = f.RemoveDuplicatePoints()
+                p, o, v, want = O.fusion_remove_duplicates(ims, *cloud)
+            assert removed == want
+            cloud = _cloud(f)
+            _same_cloud(cloud, (p, o, v))
+
+
+def test_cleanup_of_an_empty_cloud():
+    scene = syn.planes_scene(seed=3, width=40, height=30, focal=32.0, num_src=2)
+    ims, ov = syn.fusion_inputs(scene, seed=1)
+    with StereoFusion(FusionOptions(min_num_pixels=10000), ims, ov) as f:
+        f.Run()
+        assert f.RemoveDuplicatePoints() == 0 and f.RemoveOutliers() == 0
+        assert len(f.GetFusedPoints()) == 0
