@@ -92,8 +92,9 @@ int smvs_test_fusion_caps(int closure_cap, int replay_cap, int replay_stack);
 int smvs_test_fusion_paths(int in_place, int walk);
 
 /* With profiling on during smvs_fusion_run: per fused image (in fusion order)
- * the longest chain of seeds that each waited for the previous one (the
- * number of sequential replay steps the image needed) and, optionally, the
+ * the longest chain of seeds that each waited for the previous one to run (the
+ * number of sequential replay steps the image needed; a seed whose pixel another
+ * one fused does not run and takes no part) and, optionally, the
  * shear K of its ticket order (key = column + K x row of the seed grid). */
 int smvs_test_fusion_chains(smvs_fusion* f, uint32_t* chains, uint32_t* shears, int capacity, int* count);
 

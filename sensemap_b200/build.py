@@ -26,6 +26,9 @@ NVCC_FLAGS = COMMON_FLAGS + ["--use_fast_math"]
 # flush to zero): the cross-view filter's decisions and medians, and the
 # depth tests of the initial maps, the fusion's consistency tests and medians.
 EXACT_FLAGS = COMMON_FLAGS + ["-fmad=false", "-prec-div=true", "-prec-sqrt=true", "-ftz=false"]
+# Host units: loops and jump targets aligned, so that the triangulation's time does not
+# depend on where the link puts it (1.5 % between two links of one object file).
+HOST_FLAGS = NVCC_FLAGS + ["-Xcompiler", "-falign-loops=16,-falign-jumps=16"]
 EXACT_UNITS = {"smvs_cross_filter.cu", "smvs_init_maps.cu", "smvs_fusion.cu", "smvs_pyramid.cu", "smvs_prior.cu"}
 
 
@@ -54,7 +57,7 @@ def needs_build() -> bool:
 
 def _compile(src: Path, nvcc: str) -> tuple[Path, str]:
     obj = BUILD_DIR / (src.name + ".o")
-    flags = EXACT_FLAGS if src.name in EXACT_UNITS else NVCC_FLAGS
+    flags = HOST_FLAGS if src.suffix == ".cpp" else EXACT_FLAGS if src.name in EXACT_UNITS else NVCC_FLAGS
     cmd = [nvcc, *flags, *ARCH_FLAGS, "-c", str(src), "-o", str(obj)]
     res = subprocess.run(cmd, capture_output=True, text=True)
     if res.returncode != 0:
