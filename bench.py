@@ -764,6 +764,8 @@ def main():
             "kernel": (f"SweepKernelL<{RADIUS},{STEP},{12 if NSRC <= 12 else 16}>" if tune["threads_per_pixel"] == 1
                        else f"SweepKernel<{RADIUS},{STEP},{tune['threads_per_pixel']}>"),
             "taps_per_launch": taps_per_launch, "flop_per_tap": FLOP_PER_TAP, "avg_launch_ms": sweep_avg_s * 1000.0,
+            "taps_model": "nominal: every hypothesis on every view; refinement hypotheses that have lost are not sampled "
+                          "on all of them",
             "peak_source": (f"measured in this process: FP32 FMA {fp32 / 1e12:.1f} TFLOP/s, bilinear texture "
                             f"{tex / 1e9:.0f} Gsample/s; peak = min(FP32/25, texture) taps/s x 25 flop"),
             "kernel_share": {k: round(v[1] / sum(x[1] for x in prof.values()), 4) for k, v in prof.items()}}
@@ -1287,7 +1289,7 @@ def run_fusion(args):
     out_s = time.perf_counter() - t
     cleanup = {"points_fused": npts, "duplicates_removed": dup, "duplicate_pass_ms": 1000.0 * dup_s,
                "outliers_removed": outl, "outlier_pass_ms": 1000.0 * out_s,
-               "outlier_pass": "exact 6-nearest-neighbour spacing on the GPU, score histogram on the host"}
+               "outlier_pass": "exact 6-nearest-neighbour spacing, scores and histogram on the GPU"}
     f.close()
     peaks = json.loads((ROOT / "MEASURED_PEAKS.json").read_text()) if (ROOT / "MEASURED_PEAKS.json").exists() else {}
     hbm = peaks.get("hbm_gbs", 6650.0)
