@@ -165,7 +165,7 @@ __device__ __forceinline__ void FoldRange(uint32_t lo, uint32_t hi, Status* st) 
 // A lane projects a point each, then the warp writes the points' windows one
 // after another, a lane a pixel: neighbouring lanes touch neighbouring pixels. A
 // stored key only ever falls, so one that is not above the point's needs no atomic;
-// the read costs less than the atomic that it saves. Bound by its accesses to the
+// the read costs less than the atomic that it saves. Bound by the latency of the
 // L2; 400,000 points into 1600x1200 (49 pixels each): 47 us, the whole call 126 us
 // (201 us with a thread and 49 atomics a point).
 __global__ void __launch_bounds__(kThreads) SparseSplatKernel(Cam c, const float* __restrict__ xyz, size_t n,
@@ -469,7 +469,8 @@ __device__ __forceinline__ bool Window(const Cam& c, const float* __restrict__ x
 // neighbouring slots. The group is the power of two that holds a window (kSide 0,
 // any window: a warp, in several steps). `per` points a group, at most kGroup: fewer
 // where the points are too few to fill the GPU. 400,000 points into 1600x1200 with
-// ws 4, 25 slots each: 47 us, bound by its accesses to the L2; the two passes of a
+// ws 4, 25 slots each: 47 us, bound by the latency of its accesses to the L2 (64
+// registers for four windows in flight; 40, or fewer windows, took longer); the two passes of a
 // thread a point, two atomics a slot in the first, took 178 us, and the whole call
 // 358 us, now 126 us.
 template <int kGroup, int kSide>
