@@ -162,8 +162,9 @@ typedef struct smvs_problem {
 
 typedef struct smvs_engine smvs_engine;
 
-/* Device pointers to an engine's maps (valid until smvs_destroy). Layouts are
- * dense row-major; normal and cost are planar (slice-major), like GpuMat's
+/* Device pointers to an engine's maps (valid until smvs_destroy). Each is a
+ * cudaMalloc allocation of its own: other streams, peer devices and, through
+ * cudaIpcGetMemHandle, other processes may read it. Layouts are dense row-major; normal and cost are planar (slice-major), like GpuMat's
  * slices (src/util/gpu_mat.h:194-198) without the pitch. */
 typedef struct smvs_device_maps {
   int width, height, num_src;
@@ -460,9 +461,9 @@ int smvs_cross_filter_synchronize(smvs_cross_filter* cf);
 void smvs_cross_filter_destroy(smvs_cross_filter* cf);
 /* Cross filters, depth-map pools (views, kept maps, job state), fusion and
  * the initial-map builders allocate from a per-device stream-ordered memory
- * pool that keeps freed memory reserved for the next call; engines allocate
- * from a second one that keeps at most 4 GiB. This returns the free part of
- * both to the device (synchronises the device). gpu_index -1 = current
+ * pool that keeps freed memory reserved for the next call; closed engines
+ * leave at most 4 GiB of theirs to the next engine. This returns what is free
+ * of both to the device (synchronises the device). gpu_index -1 = current
  * device. */
 int smvs_cross_filter_release_cache(int gpu_index);
 

@@ -47,6 +47,7 @@
 extern "C" void smvs_internal_set_error(const char* msg);
 void smvs_internal_pose_record(const smvs_view* ref, const smvs_view* src, float* out43);
 cudaMemPool_t smvs_internal_engine_pool(int device);
+bool smvs_internal_release_map_blocks(int device);
 
 namespace {
 
@@ -974,6 +975,7 @@ int smvs_cross_filter_release_cache(int gpu_index) {
   CF_CUDA(cudaDeviceSynchronize());
   CF_CUDA(cudaMemPoolTrimTo(pool, 0));
   if (cudaMemPool_t engines = smvs_internal_engine_pool(dev)) CF_CUDA(cudaMemPoolTrimTo(engines, 0));
+  smvs_internal_release_map_blocks(dev);
   return SMVS_OK;
 }
 

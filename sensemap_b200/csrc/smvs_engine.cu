@@ -7,9 +7,11 @@
 // after every launch, src/util/cudacc.cc:50-64), per-view pitched textures
 // instead of one layered cudaArray, and status codes instead of exit().
 #include <cmath>
+#include <atomic>
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <list>
 #include <map>
 #include <mutex>
 #include <string>
@@ -29,10 +31,10 @@ cudaMemPool_t smvs_internal_device_pool(int device);
 // map and makes some 30 allocations; cudaMalloc and cudaFree took 0.6 + 0.5 ms of
 // a 160x120 map's 2.8 ms, 8 + 7 ms at 1201x899 with 8 sources, and now and then
 // 50-240 ms (the driver maps and unmaps device memory). The pool keeps at most
-// kEngineReserve bytes between engines and returns the rest at their next
+// kPoolReserve bytes between engines and returns the rest at their next
 // synchronisation; smvs_cross_filter_release_cache returns all of it.
 cudaMemPool_t smvs_internal_engine_pool(int device) {
-  constexpr uint64_t kEngineReserve = 4ull << 30;
+  constexpr uint64_t kPoolReserve = 3ull << 30;
   static std::mutex mu;
   static std::map<int, cudaMemPool_t> pools;
   std::lock_guard<std::mutex> lock(mu);
@@ -48,13 +50,82 @@ cudaMemPool_t smvs_internal_engine_pool(int device) {
     (void)cudaGetLastError();
     return nullptr;
   }
-  uint64_t keep = kEngineReserve;
+  uint64_t keep = kPoolReserve;
   cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
   pools[device] = pool;
   return pool;
 }
 
 namespace {
+
+// Memory of the maps that smvs_get_device_maps gives out. It comes from cudaMalloc,
+// not from the pool: peers reach it after cudaDeviceEnablePeerAccess and
+// cudaIpcGetMemHandle exports it, which a pool's memory does not allow. Five
+// cudaMalloc and cudaFree calls take 0.6 ms of a 160x120 map's 1.1 ms, 4 of 21.6
+// ms at 640x480 and 18 of 248 ms at 3000x2000 with 20 sources, so the blocks of a
+// closed engine wait here for the next one, unless its maps were given out: then
+// other streams, devices or processes may still read them, and cudaFree, which
+// waits for the device, takes them. At most kMapReserve bytes a device wait, the
+// oldest are freed first; Release frees all.
+struct MapBlock {
+  int device = 0;
+  size_t bytes = 0;
+  void* p = nullptr;
+};
+
+class MapBlocks {
+ public:
+  static constexpr size_t kMapReserve = (size_t)1 << 30;
+  // The smallest waiting block of `bytes` to a quarter more.
+  bool Take(int device, size_t bytes, MapBlock* out) {
+    std::lock_guard<std::mutex> lock(mu_);
+    auto best = blocks_.end();
+    for (auto it = blocks_.begin(); it != blocks_.end(); ++it)
+      if (it->device == device && it->bytes >= bytes && it->bytes <= bytes + bytes / 4 &&
+          (best == blocks_.end() || it->bytes < best->bytes))
+        best = it;
+    if (best == blocks_.end()) return false;
+    *out = *best;
+    blocks_.erase(best);
+    return true;
+  }
+  // A block that nothing on the device uses any more.
+  void Put(const MapBlock& block) {
+    std::vector<MapBlock> drop;
+    {
+      std::lock_guard<std::mutex> lock(mu_);
+      blocks_.push_back(block);
+      size_t held = 0;
+      for (const auto& b : blocks_) held += b.device == block.device ? b.bytes : 0;
+      for (auto it = blocks_.begin(); held > kMapReserve;) {
+        if (it->device != block.device) { ++it; continue; }
+        held -= it->bytes;
+        drop.push_back(*it);
+        it = blocks_.erase(it);
+      }
+    }
+    for (const auto& b : drop) cudaFree(b.p);
+  }
+  // Frees a device's waiting blocks; whether there were any.
+  bool Release(int device) {
+    std::vector<MapBlock> drop;
+    {
+      std::lock_guard<std::mutex> lock(mu_);
+      for (auto it = blocks_.begin(); it != blocks_.end();) {
+        if (it->device != device) { ++it; continue; }
+        drop.push_back(*it);
+        it = blocks_.erase(it);
+      }
+    }
+    for (const auto& b : drop) cudaFree(b.p);
+    return !drop.empty();
+  }
+
+ private:
+  std::mutex mu_;
+  std::list<MapBlock> blocks_;  // oldest first
+};
+MapBlocks& g_map_blocks = *new MapBlocks;  // engines may close after this unit's destructors
 
 thread_local std::string g_last_error;
 
@@ -172,6 +243,8 @@ struct smvs_engine {
   int64_t launches = 0;
   smvs::JobParams jp;
   std::vector<void*> allocations;
+  std::vector<MapBlock> maps;  // what smvs_get_device_maps gives out (AllocMap)
+  mutable std::atomic<bool> maps_given{false};
   std::vector<cudaTextureObject_t> textures;
   float* d_ref = nullptr;
   float* d_ref_sum = nullptr;
@@ -222,7 +295,7 @@ struct smvs_engine {
     bool any = false;
     for (cudaMemPool_t pool : {smvs_internal_device_pool(device), mem})
       any = (pool && cudaMemPoolTrimTo(pool, 0) == cudaSuccess) || any;
-    return any;
+    return g_map_blocks.Release(device) || any;
   }
   cudaError_t Get(void** p, size_t bytes) {
     return mem ? cudaMallocFromPoolAsync(p, bytes, mem, stream) : cudaMalloc(p, bytes);
@@ -232,6 +305,19 @@ struct smvs_engine {
     if (e == cudaErrorMemoryAllocation && ReleaseReserve()) e = Get(p, bytes);
     if (e != cudaSuccess) return Fail(SMVS_ENOMEM, "device allocation of %zu bytes failed: %s", bytes, cudaGetErrorString(e));
     allocations.push_back(*p);
+    return SMVS_OK;
+  }
+  int AllocMap(void** p, size_t bytes) {
+    MapBlock block;
+    if (!g_map_blocks.Take(device, bytes, &block)) {
+      block = {device, bytes, nullptr};
+      cudaError_t e = cudaMalloc(&block.p, bytes);
+      if (e == cudaErrorMemoryAllocation && ReleaseReserve()) e = cudaMalloc(&block.p, bytes);
+      if (e != cudaSuccess)
+        return Fail(SMVS_ENOMEM, "device allocation of %zu bytes failed: %s", bytes, cudaGetErrorString(e));
+    }
+    maps.push_back(block);
+    *p = block.p;
     return SMVS_OK;
   }
   // Rows of a multiple of 512 bytes from a 512-byte boundary, as textures over
@@ -248,9 +334,12 @@ struct smvs_engine {
     int dev = 0;
     const bool other = cudaGetDevice(&dev) == cudaSuccess && dev != device;
     if (other) cudaSetDevice(device);
-    if (stream) cudaDeviceSynchronize();
+    const bool synced = stream && cudaDeviceSynchronize() == cudaSuccess;
     for (auto& t : timed) { cudaEventDestroy(t.start); cudaEventDestroy(t.stop); }
     for (auto t : textures) cudaDestroyTextureObject(t);
+    for (const auto& b : maps) {
+      if (maps_given || !synced) cudaFree(b.p); else g_map_blocks.Put(b);
+    }
     for (auto p : allocations) {
       if (mem) cudaFreeAsync(p, stream); else cudaFree(p);
     }
@@ -259,6 +348,8 @@ struct smvs_engine {
     if (other) cudaSetDevice(dev);
   }
 };
+
+bool smvs_internal_release_map_blocks(int device) { return g_map_blocks.Release(device); }
 
 namespace {
 
@@ -586,11 +677,11 @@ int smvs_create(const smvs_options* opt, const smvs_problem* prob, void* stream,
   for (int i = 0; i < N; ++i) e->has_src_depth = e->has_src_depth && prob->src[i].depth != nullptr;
 
   // State maps.
-  TRY(e->Alloc((void**)&e->d_depth, WH * sizeof(float)));
-  TRY(e->Alloc((void**)&e->d_normal, 3 * WH * sizeof(float)));
-  TRY(e->Alloc((void**)&e->d_conf, WH * sizeof(float)));
-  TRY(e->Alloc((void**)&e->d_cost, (size_t)N * WH * sizeof(float)));
-  TRY(e->Alloc((void**)&e->d_view_sel, WH * sizeof(uint32_t)));
+  TRY(e->AllocMap((void**)&e->d_depth, WH * sizeof(float)));
+  TRY(e->AllocMap((void**)&e->d_normal, 3 * WH * sizeof(float)));
+  TRY(e->AllocMap((void**)&e->d_conf, WH * sizeof(float)));
+  TRY(e->AllocMap((void**)&e->d_cost, (size_t)N * WH * sizeof(float)));
+  TRY(e->AllocMap((void**)&e->d_view_sel, WH * sizeof(uint32_t)));
   p.depth = e->d_depth; p.normal = e->d_normal; p.conf = e->d_conf; p.cost = e->d_cost; p.view_sel = e->d_view_sel;
   if (prob->ref.depth) {
     TRY(StageIn(e, prob->ref.depth, WH * sizeof(float), prob->memory, (void**)&e->d_init_depth));
@@ -843,6 +934,7 @@ int smvs_get_size(const smvs_engine* e, int* w, int* h, int* n) {
 }
 int smvs_get_device_maps(const smvs_engine* e, smvs_device_maps* m) {
   if (!e || !m) return Fail(SMVS_EINVAL, "null argument");
+  e->maps_given = true;
   m->width = e->W; m->height = e->H; m->num_src = e->N;
   m->depth = e->d_depth; m->normal = e->d_normal; m->conf = e->d_conf; m->cost = e->d_cost; m->view_sel = e->d_view_sel;
   return SMVS_OK;
