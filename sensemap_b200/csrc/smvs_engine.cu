@@ -328,13 +328,14 @@ struct smvs_engine {
     if (st == SMVS_OK) *p = reinterpret_cast<void*>((reinterpret_cast<uintptr_t>(*p) + 511) & ~(uintptr_t)511);
     return st;
   }
-  // Frees the device memory once no work on the device can still read it: other
-  // streams may use this engine's maps (smvs_get_device_maps) until it is closed.
+  // Waits for the engine's own stream only: a wait for the device would end a
+  // graph capture of another thread. Of the memory, other streams can only read
+  // the maps, once their addresses were given out; cudaFree waits for those.
   ~smvs_engine() {
     int dev = 0;
     const bool other = cudaGetDevice(&dev) == cudaSuccess && dev != device;
     if (other) cudaSetDevice(device);
-    const bool synced = stream && cudaDeviceSynchronize() == cudaSuccess;
+    const bool synced = stream && cudaStreamSynchronize(stream) == cudaSuccess;
     for (auto& t : timed) { cudaEventDestroy(t.start); cudaEventDestroy(t.stop); }
     for (auto t : textures) cudaDestroyTextureObject(t);
     for (const auto& b : maps) {

@@ -1,6 +1,7 @@
 """Where an engine's device memory comes from: what callers on other devices, in
 other processes and on other threads may do with its maps and while it closes."""
 import ctypes as C
+import threading
 
 import numpy as np
 import pytest
@@ -71,3 +72,32 @@ def test_blocks_left_to_the_next_engine_are_bounded():
     assert before - torch.cuda.mem_get_info()[0] <= (4 << 30) + (256 << 20)
     N.check(lib.smvs_cross_filter_release_cache(-1))
     assert before - torch.cuda.mem_get_info()[0] <= 256 << 20
+
+
+def test_closing_an_engine_leaves_another_threads_capture_alone():
+    x = torch.zeros(256, device="cuda")
+    engines = [_engine() for _ in range(2)]
+    engines[1].DeviceMaps()  # its maps are freed, not kept
+    torch.cuda.synchronize()
+    graph, failed = torch.cuda.CUDAGraph(), []
+
+    def close_all():
+        try:
+            for pm in engines:
+                pm.close()
+            _engine().close()
+        except Exception as error:  # noqa: BLE001
+            failed.append(error)
+
+    with torch.cuda.stream(torch.cuda.Stream()):
+        graph.capture_begin(capture_error_mode="thread_local")
+        x.add_(1)
+        thread = threading.Thread(target=close_all)
+        thread.start()
+        thread.join()
+        x.add_(1)
+        graph.capture_end()
+    assert not failed
+    graph.replay()
+    torch.cuda.synchronize()
+    assert (x == 2).all()
