@@ -134,7 +134,11 @@ inline size_t SpreadSmemBytes(int R, int S, int nb) {
 // 1.080 -> 1.097; 4 views R=5 S=1: 9,600 0.358 -> 0.127, 117,600 1.247 -> 1.125, 153,600
 // 1.375 -> 1.441; 10 views R=5 S=1: 9,600 0.711 -> 0.234, 240,000 4.248 -> 4.091. So the
 // line rises with the samples of a pixel's hypothesis.
+// Radius 4, step 2 with over 16 views stays out: its thread-per-pixel instance is
+// compiled with other roundings than all others and than the spread kernels, and a
+// map must not depend on the form (test_spread_gpu compares every instance).
 inline bool UseSpread(long long pixels, int R, int S, int nb) {
+  if (R == 4 && S == 2 && nb > 16) return false;
   const long long samples = (long long)nb * (2 * R / S + 1) * (2 * R / S + 1);
   if (samples < 100) return pixels <= 10000;
   if (samples >= 1000) return pixels <= 200000;

@@ -38,3 +38,21 @@ def test_spread_form_matches_thread_per_pixel(size, sources, window, mode):
         problem.prior_wgt = np.random.default_rng(3).random((size[1], size[0])).astype(np.float32)
     for a, b in zip(_maps(opt, problem, False), _maps(opt, problem, True)):
         np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.parametrize("sources", [4, 10, 14, 20])
+@pytest.mark.parametrize("window", [(3, 1), (5, 1), (7, 1), (3, 2), (4, 2), (5, 2), (7, 2)])
+def test_every_instance_matches_thread_per_pixel(window, sources):
+    """Every compiled window with every view bucket of the thread-per-pixel kernels
+    (8, 12, 16, 32), photometric and geometric: each is an instance of its own,
+    whose roundings the compiler could choose differently."""
+    scene = small_planes(seed=11, w=100, h=75, f=80.0, n_src=sources)
+    init = perturbed_gt(scene)
+    for geometric in (False, True):
+        problem = problem_from_scene(scene, depth_maps=[v.depth_gt for v in scene.views] if geometric else None,
+                                     normal_maps=[v.normal_gt for v in scene.views] if geometric else None,
+                                     init=init if geometric else None)
+        opt = photometric_options(scene, iters=5, window_radius=window[0], window_step=window[1],
+                                  init_depth_random=not geometric, geom_consistency=geometric)
+        for a, b in zip(_maps(opt, problem, False), _maps(opt, problem, True)):
+            np.testing.assert_array_equal(a, b)
