@@ -61,6 +61,12 @@ int smvs_test_tile_waits(smvs_engine* eng, int polls, int skip_copy);
  * tiles. Maps do not change. */
 int smvs_test_persistent_grid(int max_blocks);
 
+/* The form of the checkerboard kernels that runs and pool steps of this thread
+ * take where one thread per pixel, no persistent grid and no prior leave a choice:
+ * 0 by the size of the launch, 1 the one that spreads a pixel over a block's warps,
+ * 2 one thread per pixel. Maps do not change. */
+int smvs_test_sweep_form(int form);
+
 /* The propagate-depth initial maps of an engine created with propagate_depth:
  * the given reference maps with the projected source depths composited in
  * (depth W*H, normal 3*W*H planar) and the prior depth (W*H), before random

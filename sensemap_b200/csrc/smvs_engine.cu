@@ -1000,6 +1000,12 @@ int smvs_test_persistent_grid(int max_blocks) {
   return SMVS_OK;
 }
 
+int smvs_test_sweep_form(int form) {
+  if (form < 0 || form > 2) return Fail(SMVS_EINVAL, "sweep form: bad arguments");
+  smvs::SetSweepForm(form);
+  return SMVS_OK;
+}
+
 int smvs_test_tile_waits(smvs_engine* e, int polls, int skip_copy) {
   if (!e || polls < 0) return Fail(SMVS_EINVAL, "tile waits: bad arguments");
   e->tma_polls = polls;

@@ -375,6 +375,10 @@ static std::atomic<int> g_persistent_grid_cap{0};
 int PersistentGridCap() { return g_persistent_grid_cap.load(std::memory_order_relaxed); }
 void SetPersistentGridCap(int max_blocks) { g_persistent_grid_cap.store(max_blocks, std::memory_order_relaxed); }
 
+static thread_local int t_sweep_form = 0;
+int SweepForm() { return t_sweep_form; }
+void SetSweepForm(int form) { t_sweep_form = form; }
+
 int FitThreadsPerPixel(int R, int nb, int bx, int tpp) {
   for (int t = tpp; t <= 4; t *= 2)
     if (ValidSweepShape(bx, t) && SweepKernelSmem(R, nb, bx, t) <= kMaxDynamicSmem &&

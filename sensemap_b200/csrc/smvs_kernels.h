@@ -137,8 +137,11 @@ inline size_t SpreadSmemBytes(int R, int S, int nb) {
 // Radius 4, step 2 with over 16 views stays out: its thread-per-pixel instance is
 // compiled with other roundings than all others and than the spread kernels, and a
 // map must not depend on the form (test_spread_gpu compares every instance).
+int SweepForm();  // test hook: 0 this rule, 1 the spread form at any size, 2 one thread per pixel
+void SetSweepForm(int form);
 inline bool UseSpread(long long pixels, int R, int S, int nb) {
   if (R == 4 && S == 2 && nb > 16) return false;
+  if (SweepForm() != 0) return SweepForm() == 1;
   const long long samples = (long long)nb * (2 * R / S + 1) * (2 * R / S + 1);
   if (samples < 100) return pixels <= 10000;
   if (samples >= 1000) return pixels <= 200000;
