@@ -1751,6 +1751,7 @@ struct smvs_fusion {
   uint8_t* d_trav = nullptr;
   float4* d_pix = nullptr;    // 2 per pixel (FMaps::pix)
   uint32_t* d_proj = nullptr; // FMaps::proj, when it fits
+  float* d_depth_in = nullptr;  // the depth map that is being taken in (during create)
   int deg = 0;                // overlapping images of the image that has most
   bool walk = false;          // test hook: the replay walks the claims
   uint8_t* d_rgb = nullptr;
@@ -1862,7 +1863,7 @@ void FreeAll(smvs_fusion* f) {
   Harvest(f);
   if (f->pool) {
     Free(f, f->d_views); Free(f, f->d_ov); Free(f, f->d_trav);
-    Free(f, f->d_pix); Free(f, f->d_proj);
+    Free(f, f->d_pix); Free(f, f->d_proj); Free(f, f->d_depth_in);
     Free(f, f->d_rgb); Free(f, f->d_mask);
     Free(f, f->d_claim_cnt); Free(f, f->d_claim_off); Free(f, f->d_claim_list);
     Free(f, f->d_pool); Free(f, f->d_rec_off); Free(f, f->d_over_list); Free(f, f->d_seq);
@@ -2851,17 +2852,16 @@ int smvs_fusion_create(const smvs_fusion_options* opt, const smvs_fusion_view* v
       cudaMemsetAsync(f->d_stats, 0, 3 * sizeof(uint32_t), f->stream) != cudaSuccess)
     return fail(Fail(SMVS_ECUDA, "fusion: upload failed"));
   // Maps and point maps.
+  if ((st = Alloc(f, &f->d_depth_in, (size_t)max_px))) return fail(st);
   const cudaMemcpyKind kind = memory == SMVS_MEM_HOST ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToDevice;
   for (int v = 0; v < num_views; ++v) {
     if (!f->used[v]) continue;
     const FView& hv = f->h_views[v];
     const size_t plane = (size_t)hv.W * hv.H;
-    float* d_depth = const_cast<float*>(views[v].depth);
-    if (memory == SMVS_MEM_HOST) {
-      if ((st = Alloc(f, &d_depth, plane))) return fail(st);
-      if (cudaMemcpyAsync(d_depth, views[v].depth, plane * 4, kind, f->stream) != cudaSuccess)
-        return fail(Fail(SMVS_ECUDA, "fusion: depth map copy failed"));
-    }
+    // A copy of a device map too: it takes an address of any alignment and a map on
+    // another device, which the kernel could not read.
+    if (cudaMemcpyAsync(f->d_depth_in, views[v].depth, plane * 4, kind, f->stream) != cudaSuccess)
+      return fail(Fail(SMVS_ECUDA, "fusion: depth map copy failed"));
     if (views[v].color &&
         cudaMemcpyAsync(f->d_rgb + 3ull * hv.base, views[v].color, plane * 3, kind, f->stream) != cudaSuccess)
       return fail(Fail(SMVS_ECUDA, "fusion: color copy failed"));
@@ -2877,19 +2877,17 @@ int smvs_fusion_create(const smvs_fusion_options* opt, const smvs_fusion_view* v
     }
     const float* R = views[v].R;
     PointMapKernel<<<Blocks(plane, 256), 256, 0, f->stream>>>(
-        hv, R[0], R[1], R[2], R[3], R[4], R[5], R[6], R[7], R[8], d_depth, d_normal, c.with_normal,
+        hv, R[0], R[1], R[2], R[3], R[4], R[5], R[6], R[7], R[8], f->d_depth_in, d_normal, c.with_normal,
         views[v].color != nullptr, f->d_pix, f->d_rgb);
     ++f->launches;
     if (f->d_proj) {
       ProjectTableKernel<<<Blocks(plane, 256), 256, 0, f->stream>>>(Maps(f), v, f->d_proj);
       ++f->launches;
     }
-    if (memory == SMVS_MEM_HOST) {
-      Free(f, d_depth);
-      Free(f, d_normal);
-    }
+    if (memory == SMVS_MEM_HOST) Free(f, d_normal);
     if (cudaGetLastError() != cudaSuccess) return fail(Fail(SMVS_ECUDA, "fusion: point map launch failed"));
   }
+  Free(f, f->d_depth_in);
   // The caller's maps are not referenced after this point.
   if (cudaStreamSynchronize(f->stream) != cudaSuccess) return fail(Fail(SMVS_ECUDA, "fusion: upload failed"));
   // Replay grid: every block resident.
