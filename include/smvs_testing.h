@@ -61,6 +61,11 @@ int smvs_test_tile_waits(smvs_engine* eng, int polls, int skip_copy);
  * tiles. Maps do not change. */
 int smvs_test_persistent_grid(int max_blocks);
 
+/* Device allocations of the library on this thread report that the device is full
+ * while what closed engines left to the next engine is more than held_bytes
+ * (0 restores the device's own answer). */
+int smvs_test_device_full(size_t held_bytes);
+
 /* The form of the checkerboard kernels that runs and pool steps of this thread
  * take where one thread per pixel, no persistent grid and no prior leave a choice:
  * 0 by the size of the launch, 1 the one that spreads a pixel over a block's warps,

@@ -46,8 +46,8 @@
 
 extern "C" void smvs_internal_set_error(const char* msg);
 void smvs_internal_pose_record(const smvs_view* ref, const smvs_view* src, float* out43);
-cudaMemPool_t smvs_internal_engine_pool(int device);
-bool smvs_internal_release_map_blocks(int device);
+cudaError_t smvs_internal_alloc(void** p, size_t bytes, cudaMemPool_t pool, cudaStream_t stream);
+bool smvs_internal_release_engine_reserve(int device);
 
 namespace {
 
@@ -489,8 +489,7 @@ void Harvest(smvs_cross_filter* f) {
 
 template <typename T>
 int PoolAlloc(smvs_cross_filter* f, T** p, size_t bytes) {
-  cudaError_t err = cudaMallocFromPoolAsync(reinterpret_cast<void**>(p), std::max<size_t>(bytes, 16), f->pool,
-                                            f->stream);
+  cudaError_t err = smvs_internal_alloc(reinterpret_cast<void**>(p), std::max<size_t>(bytes, 16), f->pool, f->stream);
   if (err != cudaSuccess) {
     *p = nullptr;
     return Fail(SMVS_ENOMEM, "cross filter: device allocation of %zu bytes: %s", bytes, cudaGetErrorString(err));
@@ -974,8 +973,7 @@ int smvs_cross_filter_release_cache(int gpu_index) {
   if (!pool) return Fail(SMVS_ECUDA, "no memory pool on device %d", dev);
   CF_CUDA(cudaDeviceSynchronize());
   CF_CUDA(cudaMemPoolTrimTo(pool, 0));
-  if (cudaMemPool_t engines = smvs_internal_engine_pool(dev)) CF_CUDA(cudaMemPoolTrimTo(engines, 0));
-  smvs_internal_release_map_blocks(dev);
+  smvs_internal_release_engine_reserve(dev);
   return SMVS_OK;
 }
 

@@ -56,7 +56,14 @@ cudaMemPool_t smvs_internal_engine_pool(int device) {
   return pool;
 }
 
+// Gives a device back what closed engines hold of it; false: nothing was tried.
+bool smvs_internal_release_engine_reserve(int device);
+
 namespace {
+
+// Test hook (smvs_test_device_full): what closed engines may hold of the device
+// before this thread's allocations report that it is full; 0: off.
+thread_local size_t t_full_above = 0;
 
 // Memory of the maps that smvs_get_device_maps gives out. It comes from cudaMalloc,
 // not from the pool: peers reach it after cudaDeviceEnablePeerAccess and
@@ -120,12 +127,36 @@ class MapBlocks {
     for (const auto& b : drop) cudaFree(b.p);
     return !drop.empty();
   }
+  size_t Held(int device) {
+    std::lock_guard<std::mutex> lock(mu_);
+    size_t held = 0;
+    for (const auto& b : blocks_) held += b.device == device ? b.bytes : 0;
+    return held;
+  }
 
  private:
   std::mutex mu_;
   std::list<MapBlock> blocks_;  // oldest first
 };
 MapBlocks& g_map_blocks = *new MapBlocks;  // engines may close after this unit's destructors
+
+// What closed engines hold of a device: the pool's free part and the map blocks.
+size_t EngineReserve(int device) {
+  uint64_t reserved = 0, used = 0;
+  cudaMemPool_t pool = smvs_internal_engine_pool(device);
+  if (pool && (cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &reserved) != cudaSuccess ||
+               cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) != cudaSuccess))
+    reserved = used = 0;
+  return (size_t)(reserved - used) + g_map_blocks.Held(device);
+}
+
+// Device memory from `pool` in stream order, without one from cudaMalloc.
+cudaError_t DeviceAlloc(void** p, size_t bytes, cudaMemPool_t pool, cudaStream_t stream) {
+  int dev = 0;
+  if (t_full_above > 0 && cudaGetDevice(&dev) == cudaSuccess && EngineReserve(dev) > t_full_above)
+    return cudaErrorMemoryAllocation;
+  return pool ? cudaMallocFromPoolAsync(p, bytes, pool, stream) : cudaMalloc(p, bytes);
+}
 
 thread_local std::string g_last_error;
 
@@ -232,6 +263,23 @@ cudaError_t MakeTexture(void* ptr, int storage_or_float, int w, int h, size_t pi
 
 }  // namespace
 
+bool smvs_internal_release_engine_reserve(int device) {
+  cudaMemPool_t pool = smvs_internal_engine_pool(device);
+  const bool trimmed = pool && cudaMemPoolTrimTo(pool, 0) == cudaSuccess;
+  return g_map_blocks.Release(device) || trimmed;
+}
+
+// The allocations of everything but engines (these also return what the library's
+// other pool holds): what closed engines hold goes back to the current device
+// before one reports that the device is full.
+cudaError_t smvs_internal_alloc(void** p, size_t bytes, cudaMemPool_t pool, cudaStream_t stream) {
+  cudaError_t e = DeviceAlloc(p, bytes, pool, stream);
+  int dev = 0;
+  if (e != cudaErrorMemoryAllocation || cudaGetDevice(&dev) != cudaSuccess) return e;
+  (void)cudaGetLastError();
+  return smvs_internal_release_engine_reserve(dev) ? DeviceAlloc(p, bytes, pool, stream) : e;
+}
+
 struct smvs_engine {
   int device = 0;
   cudaStream_t stream = nullptr;
@@ -292,17 +340,13 @@ struct smvs_engine {
   bool ReleaseReserve() {
     (void)cudaGetLastError();
     if (cudaDeviceSynchronize() != cudaSuccess) return false;
-    bool any = false;
-    for (cudaMemPool_t pool : {smvs_internal_device_pool(device), mem})
-      any = (pool && cudaMemPoolTrimTo(pool, 0) == cudaSuccess) || any;
-    return g_map_blocks.Release(device) || any;
-  }
-  cudaError_t Get(void** p, size_t bytes) {
-    return mem ? cudaMallocFromPoolAsync(p, bytes, mem, stream) : cudaMalloc(p, bytes);
+    cudaMemPool_t pool = smvs_internal_device_pool(device);
+    const bool trimmed = pool && cudaMemPoolTrimTo(pool, 0) == cudaSuccess;
+    return smvs_internal_release_engine_reserve(device) || trimmed;
   }
   int Alloc(void** p, size_t bytes) {
-    cudaError_t e = Get(p, bytes);
-    if (e == cudaErrorMemoryAllocation && ReleaseReserve()) e = Get(p, bytes);
+    cudaError_t e = DeviceAlloc(p, bytes, mem, stream);
+    if (e == cudaErrorMemoryAllocation && ReleaseReserve()) e = DeviceAlloc(p, bytes, mem, stream);
     if (e != cudaSuccess) return Fail(SMVS_ENOMEM, "device allocation of %zu bytes failed: %s", bytes, cudaGetErrorString(e));
     allocations.push_back(*p);
     return SMVS_OK;
@@ -311,8 +355,8 @@ struct smvs_engine {
     MapBlock block;
     if (!g_map_blocks.Take(device, bytes, &block)) {
       block = {device, bytes, nullptr};
-      cudaError_t e = cudaMalloc(&block.p, bytes);
-      if (e == cudaErrorMemoryAllocation && ReleaseReserve()) e = cudaMalloc(&block.p, bytes);
+      cudaError_t e = DeviceAlloc(&block.p, bytes, nullptr, nullptr);
+      if (e == cudaErrorMemoryAllocation && ReleaseReserve()) e = DeviceAlloc(&block.p, bytes, nullptr, nullptr);
       if (e != cudaSuccess)
         return Fail(SMVS_ENOMEM, "device allocation of %zu bytes failed: %s", bytes, cudaGetErrorString(e));
     }
@@ -349,8 +393,6 @@ struct smvs_engine {
     if (other) cudaSetDevice(dev);
   }
 };
-
-bool smvs_internal_release_map_blocks(int device) { return g_map_blocks.Release(device); }
 
 namespace {
 
@@ -997,6 +1039,11 @@ void smvs_destroy(smvs_engine* e) { delete e; }
 int smvs_test_persistent_grid(int max_blocks) {
   if (max_blocks < 0) return Fail(SMVS_EINVAL, "persistent grid: bad arguments");
   smvs::SetPersistentGridCap(max_blocks);
+  return SMVS_OK;
+}
+
+int smvs_test_device_full(size_t held_bytes) {
+  t_full_above = held_bytes;
   return SMVS_OK;
 }
 

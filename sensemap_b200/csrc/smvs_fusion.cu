@@ -45,6 +45,7 @@
 
 extern "C" void smvs_internal_set_error(const char* msg);
 cudaMemPool_t smvs_internal_device_pool(int device);
+cudaError_t smvs_internal_alloc(void** p, size_t bytes, cudaMemPool_t pool, cudaStream_t stream);
 
 namespace {
 
@@ -1845,7 +1846,7 @@ void Harvest(smvs_fusion* f) {
 template <typename T>
 int Alloc(smvs_fusion* f, T** p, size_t count) {
   const size_t bytes = std::max<size_t>(count * sizeof(T), 16);
-  cudaError_t err = cudaMallocFromPoolAsync(reinterpret_cast<void**>(p), bytes, f->pool, f->stream);
+  cudaError_t err = smvs_internal_alloc(reinterpret_cast<void**>(p), bytes, f->pool, f->stream);
   if (err != cudaSuccess) {
     *p = nullptr;
     return Fail(SMVS_ENOMEM, "fusion: device allocation of %zu bytes: %s", bytes, cudaGetErrorString(err));

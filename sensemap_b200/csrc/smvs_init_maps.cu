@@ -36,6 +36,7 @@
 
 extern "C" void smvs_internal_set_error(const char* msg);
 cudaMemPool_t smvs_internal_device_pool(int device);
+cudaError_t smvs_internal_alloc(void** p, size_t bytes, cudaMemPool_t pool, cudaStream_t stream);
 
 namespace smvs {
 // smvs_delaunay.cpp
@@ -713,7 +714,7 @@ struct Call {
   template <typename T>
   int Alloc(T** p, size_t bytes) {
     if (nblocks == (int)(sizeof(blocks) / sizeof(blocks[0]))) return Fail(SMVS_ENOMEM, "init maps: too many buffers");
-    cudaError_t e = cudaMallocFromPoolAsync(reinterpret_cast<void**>(p), std::max<size_t>(bytes, 16), pool, stream);
+    cudaError_t e = smvs_internal_alloc(reinterpret_cast<void**>(p), std::max<size_t>(bytes, 16), pool, stream);
     if (e != cudaSuccess) return Fail(SMVS_ENOMEM, "init maps: device allocation of %zu bytes: %s", bytes,
                                       cudaGetErrorString(e));
     blocks[nblocks++] = *p;

@@ -34,6 +34,7 @@ extern "C" void smvs_internal_set_error(const char* msg);
 int smvs_internal_prepare_job(smvs::JobParams* p, const smvs_options* o);
 void smvs_internal_pose_record(const smvs_view* ref, const smvs_view* src, float* out43);
 cudaMemPool_t smvs_internal_device_pool(int device);
+cudaError_t smvs_internal_alloc(void** p, size_t bytes, cudaMemPool_t pool, cudaStream_t stream);
 
 namespace {
 
@@ -46,7 +47,7 @@ namespace {
 // kernel that may read it; without a memory pool the plain allocator is used.
 cudaError_t DevMalloc(cudaMemPool_t mem, cudaStream_t s, void** p, size_t bytes) {
   *p = nullptr;
-  return mem ? cudaMallocFromPoolAsync(p, bytes, mem, s) : cudaMalloc(p, bytes);
+  return smvs_internal_alloc(p, bytes, mem, s);
 }
 void DevFree(cudaMemPool_t mem, cudaStream_t s, void* p) {
   if (!p) return;
@@ -380,9 +381,9 @@ int EnsureCapacity(smvs_pool* P, int n) {
   }
   P->d_jobs = nullptr; P->d_ints = nullptr; P->h_jobs = nullptr; P->h_ints = nullptr;
   P->d_maps = nullptr; P->h_maps = nullptr;
-  POOL_CUDA(cudaMalloc(&P->d_jobs, sizeof(smvs::JobParams) * cap));
-  POOL_CUDA(cudaMalloc(&P->d_ints, sizeof(int) * IntsSize(cap)));
-  POOL_CUDA(cudaMalloc(&P->d_maps, sizeof(CUtensorMap) * cap));
+  POOL_CUDA(smvs_internal_alloc((void**)&P->d_jobs, sizeof(smvs::JobParams) * cap, nullptr, nullptr));
+  POOL_CUDA(smvs_internal_alloc((void**)&P->d_ints, sizeof(int) * IntsSize(cap), nullptr, nullptr));
+  POOL_CUDA(smvs_internal_alloc((void**)&P->d_maps, sizeof(CUtensorMap) * cap, nullptr, nullptr));
   for (int i = 0; i < 2; ++i) {
     POOL_CUDA(cudaMallocHost(&P->h_jobs_set[i], sizeof(smvs::JobParams) * cap));
     POOL_CUDA(cudaMallocHost(&P->h_ints_set[i], sizeof(int) * IntsSize(cap)));
@@ -449,7 +450,7 @@ int smvs_pool_create(const smvs_pool_options* o, void* stream, smvs_pool** out) 
   P->arena.stream = P->stream;
   int st = EnsureCapacity(P, o->max_active_jobs);
   if (st) { delete P; return st; }
-  if (cudaMalloc(&P->d_status, sizeof(int)) != cudaSuccess ||
+  if (smvs_internal_alloc((void**)&P->d_status, sizeof(int), nullptr, nullptr) != cudaSuccess ||
       cudaMemsetAsync(P->d_status, 0, sizeof(int), P->stream) != cudaSuccess ||
       cudaMallocHost(&P->h_status, sizeof(int)) != cudaSuccess) {
     delete P;

@@ -8,8 +8,14 @@ import pytest
 import torch
 
 from sensemap_b200 import _native as N
-from sensemap_b200.patch_match import PatchMatchACMMCuda, Problem, View
-from tests.helpers import photometric_options, problem_from_scene, small_planes
+from sensemap_b200 import synthetic as syn
+from sensemap_b200.cross_filter import CrossFilterCuda
+from sensemap_b200.fusion import FusionOptions, StereoFusion
+from sensemap_b200.init_maps import init_depth_from_sparse_points
+from sensemap_b200.patch_match import PatchMatchACMMCuda, PatchMatchOptions, Problem, View
+from sensemap_b200.pool import DepthMapPool
+from tests.helpers import (filter_api_inputs, filter_set, photometric_options, problem_from_scene,
+                           small_planes)
 
 pytestmark = pytest.mark.gpu
 
@@ -101,3 +107,53 @@ def test_closing_an_engine_leaves_another_threads_capture_alone():
     graph.replay()
     torch.cuda.synchronize()
     assert (x == 2).all()
+
+
+def _fusion():
+    scene = syn.planes_scene(seed=3, width=90, height=70, focal=72.0, num_src=3)
+    images, overlaps = syn.fusion_inputs(scene, seed=1)
+    with StereoFusion(FusionOptions(), images, overlaps) as f:
+        f.Run()
+        assert f.RemoveOutliers() >= 0
+
+
+def _cross_filter():
+    _, views, problems = filter_set(n_views=3, w=64, h=48)
+    cf = CrossFilterCuda(PatchMatchOptions(), *filter_api_inputs(views, problems))
+    cf.Run()
+    cf.close()
+
+
+def _initial_map():
+    scene = small_planes(seed=11, w=64, h=48)
+    v = scene.views[0]
+    init_depth_from_sparse_points(64, 48, v.K, v.R, v.T, np.random.default_rng(0).random((50, 3)))
+
+
+def _pool():
+    scene = small_planes(seed=11, w=64, h=48)
+    with DepthMapPool(max_active_jobs=2) as pool:
+        for i, v in enumerate(scene.views):
+            pool.add_view(i, View(v.image, v.K, v.R, v.T))
+        job = pool.submit(photometric_options(scene, iters=1), 0, [1, 2, 3, 4])
+        pool.run_until_done([job])
+        pool.keep_maps(job)
+
+
+def _next_engine():
+    _engine(w=64, h=48).close()
+
+
+@pytest.mark.parametrize("call", [_fusion, _cross_filter, _initial_map, _pool, _next_engine])
+def test_a_full_device_takes_back_what_closed_engines_left(call):
+    """An engine of 1600x1200 leaves over 64 MiB to the next one; on a device that
+    is full as long as it does, every kind of call gets its memory all the same."""
+    lib = N.lib()
+    scene = small_planes(w=32, h=24)
+    views = [View(np.zeros((1200, 1600), np.uint8), v.K, v.R, v.T) for v in scene.views]
+    PatchMatchACMMCuda(photometric_options(scene, iters=0), Problem(0, [1, 2, 3, 4], views)).close()
+    N.check(lib.smvs_test_device_full(64 << 20))
+    try:
+        call()
+    finally:
+        N.check(lib.smvs_test_device_full(0))
