@@ -65,6 +65,9 @@ int smvs_test_persistent_grid(int max_blocks);
  * while what closed engines left to the next engine is more than held_bytes
  * (0 restores the device's own answer). */
 int smvs_test_device_full(size_t held_bytes);
+/* The nth device allocation that this thread asks for from now on, of anything but
+ * an engine, reports that the device is full (0: none). */
+int smvs_test_fail_allocation(int nth);
 
 /* The form of the checkerboard kernels that runs and pool steps of this thread
  * take where one thread per pixel, no persistent grid and no prior leave a choice:

@@ -261,6 +261,7 @@ _SIGNATURES = {
     "smvs_test_tile_waits": (C.c_int, [C.c_void_p, C.c_int, C.c_int]),
     "smvs_test_persistent_grid": (C.c_int, [C.c_int]),
     "smvs_test_device_full": (C.c_int, [C.c_size_t]),
+    "smvs_test_fail_allocation": (C.c_int, [C.c_int]),
     "smvs_test_sweep_form": (C.c_int, [C.c_int]),
     "smvs_test_propagate_init": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p]),
     "smvs_test_delaunay": (C.c_int, [C.c_void_p, C.c_int, C.c_void_p, C.c_int, C.POINTER(C.c_int)]),

@@ -64,6 +64,9 @@ namespace {
 // Test hook (smvs_test_device_full): what closed engines may hold of the device
 // before this thread's allocations report that it is full; 0: off.
 thread_local size_t t_full_above = 0;
+// Test hook (smvs_test_fail_allocation): the smvs_internal_alloc call that fails,
+// counted down; 0: off.
+thread_local int t_fail_at = 0;
 
 // Memory of the maps that smvs_get_device_maps gives out. It comes from cudaMalloc,
 // not from the pool: peers reach it after cudaDeviceEnablePeerAccess and
@@ -273,6 +276,7 @@ bool smvs_internal_release_engine_reserve(int device) {
 // other pool holds): what closed engines hold goes back to the current device
 // before one reports that the device is full.
 cudaError_t smvs_internal_alloc(void** p, size_t bytes, cudaMemPool_t pool, cudaStream_t stream) {
+  if (t_fail_at > 0 && --t_fail_at == 0) return cudaErrorMemoryAllocation;
   cudaError_t e = DeviceAlloc(p, bytes, pool, stream);
   int dev = 0;
   if (e != cudaErrorMemoryAllocation || cudaGetDevice(&dev) != cudaSuccess) return e;
@@ -1044,6 +1048,12 @@ int smvs_test_persistent_grid(int max_blocks) {
 
 int smvs_test_device_full(size_t held_bytes) {
   t_full_above = held_bytes;
+  return SMVS_OK;
+}
+
+int smvs_test_fail_allocation(int nth) {
+  if (nth < 0) return Fail(SMVS_EINVAL, "fail allocation: bad arguments");
+  t_fail_at = nth;
   return SMVS_OK;
 }
 

@@ -1847,6 +1847,15 @@ template <typename T>
 int Alloc(smvs_fusion* f, T** p, size_t count) {
   const size_t bytes = std::max<size_t>(count * sizeof(T), 16);
   cudaError_t err = smvs_internal_alloc(reinterpret_cast<void**>(p), bytes, f->pool, f->stream);
+  if (err == cudaErrorMemoryAllocation && f->d_proj) {
+    // The closures can do without the projection table (and launch by whether it is
+    // there): it makes room first.
+    (void)cudaGetLastError();
+    cudaFreeAsync(f->d_proj, f->stream);
+    f->d_proj = nullptr;
+    if (cudaStreamSynchronize(f->stream) == cudaSuccess && cudaMemPoolTrimTo(f->pool, 0) == cudaSuccess)
+      err = smvs_internal_alloc(reinterpret_cast<void**>(p), bytes, f->pool, f->stream);
+  }
   if (err != cudaSuccess) {
     *p = nullptr;
     return Fail(SMVS_ENOMEM, "fusion: device allocation of %zu bytes: %s", bytes, cudaGetErrorString(err));
@@ -1988,7 +1997,7 @@ FPreds Preds(const smvs_fusion* f) {
   p.cnt = f->d_pred_cnt;
   p.list = f->d_pred_list;
   p.used = f->d_pred_used;
-  p.cap = f->walk ? 0ull : std::min<unsigned long long>(f->claim_list_cap, 0xffffffffull);
+  p.cap = f->walk || !f->d_pred_list ? 0ull : std::min<unsigned long long>(f->claim_list_cap, 0xffffffffull);
   p.claim_off = f->d_claim_off;
   p.claim_list = f->d_claim_list;
   return p;
@@ -2132,10 +2141,9 @@ int FuseImage(smvs_fusion* f, int image) {
       Free(f, f->d_claim_list);
       Free(f, f->d_pred_list);
       f->claim_list_cap = (size_t)claims + 1024;
-      if ((st = Alloc(f, &f->d_claim_list, f->claim_list_cap)) || (st = Alloc(f, &f->d_pred_list, f->claim_list_cap))) {
-        f->claim_list_cap = 0;
-        return st;
-      }
+      if ((st = Alloc(f, &f->d_claim_list, f->claim_list_cap))) { f->claim_list_cap = 0; return st; }
+      // Without room for the predecessor lists the replay walks the claims.
+      if (Alloc(f, &f->d_pred_list, f->claim_list_cap)) (void)cudaGetLastError();
     }
     ClaimCountKernel<<<Blocks(32 * nseeds, 256), 256, 0, f->stream>>>(Recs(f), (uint32_t)nseeds, f->d_claim_cnt);
     ++f->launches;
@@ -2819,8 +2827,10 @@ int smvs_fusion_create(const smvs_fusion_options* opt, const smvs_fusion_view* v
   // pool at that bound for the largest image (within a quarter of the free
   // device memory); it grows if an image needs more.
   int max_deg = 0;
-  for (int v = 0; v < num_views; ++v) max_deg = std::max(max_deg, overlap_offsets[v + 1] - overlap_offsets[v]);
-  f->deg = max_deg;
+  for (int v = 0; v < num_views; ++v) {
+    max_deg = std::max(max_deg, overlap_offsets[v + 1] - overlap_offsets[v]);
+    if (f->used[v]) f->deg = std::max(f->deg, overlap_offsets[v + 1] - overlap_offsets[v]);
+  }
   const double radius = std::max(opt->max_reproj_error, 0.5);
   const uint64_t disk = (uint64_t)std::ceil((2.0 * radius + 1.0) * (2.0 * radius + 1.0));
   const uint32_t cnt_est = (uint32_t)std::min<uint64_t>(kCap, disk * (uint64_t)(1 + max_deg));
@@ -2831,12 +2841,13 @@ int smvs_fusion_create(const smvs_fusion_options* opt, const smvs_fusion_view* v
   f->pool_words = (size_t)std::min<uint64_t>(std::max<uint64_t>(est, max_px * 64ull), 0xfffffff0ull);
   if ((st = Alloc(f, &f->d_pool, f->pool_words))) return fail(st);
   // The projection table: a word per pixel and overlapping image (845 MB for 11
-  // views 1600x1200), when that is at most an eighth of the free memory; else the
-  // closures project in place.
+  // views 1600x1200), when that is at most an eighth of the memory still free and
+  // can be had; else the closures project in place.
   f->walk = t_walk;
-  if (!t_in_place && max_deg > 0 && T * (size_t)max_deg * sizeof(uint32_t) <= free_b / 8 &&
-      (st = Alloc(f, &f->d_proj, T * (size_t)max_deg)))
-    return fail(st);
+  if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) free_b = 0;
+  const size_t table = T * (size_t)f->deg;
+  if (!t_in_place && table > 0 && table * sizeof(uint32_t) <= free_b / 8 && Alloc(f, &f->d_proj, table))
+    (void)cudaGetLastError();
   auto up = [&](void* dst, const void* src, size_t bytes) -> cudaError_t {
     return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDefault, f->stream);
   };
@@ -2898,8 +2909,10 @@ int smvs_fusion_create(const smvs_fusion_options* opt, const smvs_fusion_view* v
     return fail(Fail(SMVS_ECUDA, "fusion: cannot size the replay grid"));
   f->replay_blocks = per_sm * sms;
   const auto closure = f->d_proj ? ClosureKernel<true> : ClosureKernel<false>;
-  if (cudaFuncSetAttribute(closure, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kClosureSmem) != cudaSuccess ||
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, closure, 32 * kClosureWarps, kClosureSmem) !=
+  for (const auto kernel : {ClosureKernel<true>, ClosureKernel<false>})  // the table may have to go during the run
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kClosureSmem) != cudaSuccess)
+      return fail(Fail(SMVS_ECUDA, "fusion: cannot size the closure grid"));
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, closure, 32 * kClosureWarps, kClosureSmem) !=
           cudaSuccess ||
       per_sm < 1)
     return fail(Fail(SMVS_ECUDA, "fusion: cannot size the closure grid"));

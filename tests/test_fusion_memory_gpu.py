@@ -1,0 +1,67 @@
+"""Fusion on a device that runs out of memory: what it can do without goes first."""
+import numpy as np
+import pytest
+
+from sensemap_b200 import _native as N
+from sensemap_b200 import synthetic as syn
+from sensemap_b200.fusion import FusionOptions, StereoFusion
+
+pytestmark = pytest.mark.gpu
+
+
+def _inputs():
+    scene = syn.heightfield_scene(seed=9, width=96, height=72, focal=72.0, num_src=3, device="cuda")
+    return syn.fusion_inputs(scene, seed=3)
+
+
+def _fuse(images, overlaps, fail_at):
+    """The points, or None where the call reported that memory ran out."""
+    lib = N.lib()
+    N.check(lib.smvs_test_fail_allocation(fail_at))
+    try:
+        with StereoFusion(FusionOptions(), images, overlaps) as f:
+            f.Run()
+            return f.GetFusedPoints().copy()
+    except N.SmvsError as error:
+        assert error.status == N.SMVS_ENOMEM
+        return None
+    finally:
+        N.check(lib.smvs_test_fail_allocation(0))
+
+
+@pytest.mark.parametrize("in_place", [0, 1])
+def test_any_allocation_may_fail(in_place):
+    """The nth allocation fails, for every n. Once the projection table is there it
+    makes room for whatever comes after; without one, the predecessor lists can be
+    left out. No failure changes the points."""
+    images, overlaps = _inputs()
+    want = _fuse(images, overlaps, 0)
+    assert len(want) > 100
+    N.check(N.lib().smvs_test_fusion_paths(in_place, 0))
+    try:
+        failed, total = [], 70
+        for nth in range(1, total + 1):
+            got = _fuse(images, overlaps, nth)
+            if got is None:
+                failed.append(nth)
+            else:
+                np.testing.assert_array_equal(got.view(np.uint8), want.view(np.uint8))
+    finally:
+        N.check(N.lib().smvs_test_fusion_paths(0, 0))
+    before_table = 21  # the arrays of all pixels and the record pool
+    if in_place:
+        assert max(failed) > before_table + 1 and max(failed) < total
+        assert any(nth not in failed for nth in range(before_table + 1, max(failed)))
+    else:
+        assert failed == list(range(1, len(failed) + 1)) and len(failed) <= before_table
+
+
+def test_overlap_list_of_an_unused_image_costs_nothing():
+    """An image without a depth map overlaps all others many times over; the table's
+    rows keep the width of the longest list of a used image."""
+    images, overlaps = _inputs()
+    want = _fuse(images, overlaps, 0)
+    images = list(images) + [type(images[0])(K=images[0].K, R=images[0].R, T=images[0].T)]
+    overlaps = list(overlaps) + [list(range(len(overlaps))) * 200]
+    got = _fuse(images, overlaps, 0)
+    np.testing.assert_array_equal(got.view(np.uint8), want.view(np.uint8))
