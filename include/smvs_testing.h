@@ -105,6 +105,10 @@ int smvs_test_fusion_caps(int closure_cap, int replay_cap, int replay_stack);
  * replay walks the claims of a record's pixels (no predecessor lists). */
 int smvs_test_fusion_paths(int in_place, int walk);
 
+/* Rows and columns of n pixels of an image of the given width, as the closures
+ * recover them from a pixel's index (pixels below 2^31). Host only. */
+int smvs_test_row_and_column(const uint32_t* px, int n, int width, int32_t* rows, int32_t* cols);
+
 /* With profiling on during smvs_fusion_run: per fused image (in fusion order)
  * the longest chain of seeds that each waited for the previous one to run (the
  * number of sequential replay steps the image needed; a seed whose pixel another

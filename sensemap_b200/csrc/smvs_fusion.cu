@@ -223,6 +223,21 @@ __global__ void PointMapKernel(FView v, float R0, float R1, float R2, float R3, 
   }
 }
 
+// Row and column of pixel px of an image W wide. The product is at most one row off
+// below some four million rows and a few hundred at 2^31 pixels of one column.
+__host__ __device__ __forceinline__ void RowAndColumn(uint32_t px, int W, int* row, int* col) {
+#ifdef __CUDA_ARCH__
+  int r = (int)__fmul_rn((float)px, __frcp_rn((float)W));
+#else
+  int r = (int)((float)px * (1.0f / (float)W));
+#endif
+  int c = (int)(px - (uint32_t)r * (uint32_t)W);
+  while (c < 0) { c += W; --r; }
+  while (c >= W) { c -= W; ++r; }
+  *row = r;
+  *col = c;
+}
+
 // Where the pixels of image `view` fall in its overlapping images. A closure
 // asks for these places again in every seed that reaches the pixel (some 100
 // seeds in the first image of 11 views): the table replaces two divisions, nine
@@ -568,13 +583,7 @@ __global__ void __launch_bounds__(32 * kClosureWarps) ClosureKernel(FMaps m, FCo
             // pixels that fail fail it.
             if (kTable) u = m.ov[m.views[sh.vid[i]].ov_begin + k];
             const FView& fu = m.views[u];
-            if (kTable) {
-              const uint32_t px = q - fu.base;
-              row = (int)__fmul_rn((float)px, __frcp_rn((float)fu.W));  // at most one off
-              col = (int)px - row * fu.W;
-              if (col < 0) { col += fu.W; --row; }
-              if (col >= fu.W) { col -= fu.W; ++row; }
-            }
+            if (kTable) RowAndColumn(q - fu.base, fu.W, &row, &col);
             float pc, pr, pz;
             if (u < 32) {
               pc = sh.seed[0][u];
@@ -3070,6 +3079,12 @@ int smvs_test_fusion_replay_times(smvs_fusion* f, double* out, int capacity, int
     o[7] = (double)ti[7] / seeds / 1000.0;
     o[8] = (double)ti[8] / seeds / 1000.0;
   }
+  return SMVS_OK;
+}
+
+int smvs_test_row_and_column(const uint32_t* px, int n, int width, int32_t* rows, int32_t* cols) {
+  if (n < 0 || width < 1 || (n > 0 && (!px || !rows || !cols))) return Fail(SMVS_EINVAL, "row and column: bad arguments");
+  for (int i = 0; i < n; ++i) RowAndColumn(px[i], width, rows + i, cols + i);
   return SMVS_OK;
 }
 
