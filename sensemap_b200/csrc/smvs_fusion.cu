@@ -2385,18 +2385,18 @@ __global__ void __launch_bounds__(256) DupLevelsKernel(uint32_t n, const uint64_
     if (bins[k]) atomicAdd(counts + k, bins[k]);
 }
 
-// Lists the points by level: cursor[level] starts at the level's first place.
+// Lists the points by level: cursor[level] starts at the level's first place. All
+// lanes of a warp match; those past the end share a level that no point has.
 __global__ void DupOrderKernel(uint32_t n, const uint64_t* __restrict__ off, int max_level,
                                uint32_t* __restrict__ cursor, uint32_t* __restrict__ list) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const int level = (int)min(off[i + 1] - off[i], (uint64_t)max_level);
-  const unsigned same = __match_any_sync(__activemask(), level);
+  const int level = i < n ? (int)min(off[i + 1] - off[i], (uint64_t)max_level) : -1;
+  const unsigned same = __match_any_sync(0xffffffffu, level);
   const int lane = threadIdx.x % 32, leader = __ffs(same) - 1;
   uint32_t first = 0;
-  if (lane == leader) first = atomicAdd(cursor + level, (uint32_t)__popc(same));
-  first = __shfl_sync(same, first, leader);
-  list[first + __popc(same & ((1u << lane) - 1))] = i;
+  if (i < n && lane == leader) first = atomicAdd(cursor + level, (uint32_t)__popc(same));
+  first = __shfl_sync(0xffffffffu, first, leader);
+  if (i < n) list[first + __popc(same & ((1u << lane) - 1))] = i;
 }
 
 // Eigen 3.3's float evaluation of K * (R * X + T) (coefficient-based 3x3 products
