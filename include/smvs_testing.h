@@ -105,6 +105,11 @@ int smvs_test_fusion_caps(int closure_cap, int replay_cap, int replay_stack);
  * replay walks the claims of a record's pixels (no predecessor lists). */
 int smvs_test_fusion_paths(int in_place, int walk);
 
+/* The cross filter's decode of n normal codes: the quotients of each code's upper
+ * and lower half by 32767 (quotients[2i], [2i + 1]) and the normal it stands for
+ * (normals[3i..3i+2]). Device buffers; enqueued on `stream`. */
+int smvs_test_decode_codes(const uint32_t* codes, int n, float* quotients, float* normals, void* stream);
+
 /* Rows and columns of n pixels of an image of the given width, as the closures
  * recover them from a pixel's index (pixels below 2^31). Host only. */
 int smvs_test_row_and_column(const uint32_t* px, int n, int width, int32_t* rows, int32_t* cols);

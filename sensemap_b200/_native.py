@@ -276,6 +276,7 @@ _SIGNATURES = {
                                            C.c_int, C.c_int, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p]),
     "smvs_test_fusion_caps": (C.c_int, [C.c_int, C.c_int, C.c_int]),
     "smvs_test_fusion_paths": (C.c_int, [C.c_int, C.c_int]),
+    "smvs_test_decode_codes": (C.c_int, [C.c_void_p, C.c_int, C.c_void_p, C.c_void_p, C.c_void_p]),
     "smvs_test_row_and_column": (C.c_int, [C.c_void_p, C.c_int, C.c_int, C.c_void_p, C.c_void_p]),
     "smvs_test_fusion_chains": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_int, C.POINTER(C.c_int)]),
     "smvs_test_fusion_image_ms": (C.c_int, [C.c_void_p, C.c_void_p, C.c_int, C.POINTER(C.c_int)]),

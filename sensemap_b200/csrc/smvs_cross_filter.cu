@@ -43,6 +43,7 @@
 #include <cuda_runtime.h>
 
 #include "../../include/smvs.h"
+#include "../../include/smvs_testing.h"
 
 extern "C" void smvs_internal_set_error(const char* msg);
 void smvs_internal_pose_record(const smvs_view* ref, const smvs_view* src, float* out43);
@@ -140,15 +141,13 @@ __device__ __forceinline__ uint32_t Encode(float n0, float n1, float n2) {
 }
 
 // iq / 32767 in IEEE rounding for a 16-bit iq: the product with the reciprocal,
-// corrected by its exact residual (equal to the division for all 65,536 values).
-// The bits of 2^23 + iq are the float's, without a conversion.
-__host__ __device__ __forceinline__ float Over32767(uint32_t iq) {
+// corrected by its exact residual (division by a constant known in advance,
+// Brisebarre, Muller and Raina, IEEE Transactions on Computers 53(8), 2004); equal
+// to the division for all 65,536 values, which a test compares. The bits of
+// 2^23 + iq are the float's, without a conversion.
+__device__ __forceinline__ float Over32767(uint32_t iq) {
   constexpr float kInv = 1.0f / 32767.0f;
-#ifdef __CUDA_ARCH__
   const float x = __uint_as_float(0x4b000000u | iq) - 8388608.0f;
-#else
-  const float x = (float)iq;
-#endif
   const float q = x * kInv;
   return fmaf(fmaf(-32767.0f, q, x), kInv, q);
 }
@@ -249,6 +248,19 @@ __device__ __forceinline__ int2 BlockOf(const CfGrid& g) {
   const int by = b / per_band, rem = b - by * per_band;
   const int job = rem / g.blocks_x;
   return make_int2(job, by * g.blocks_x + rem - job * g.blocks_x);
+}
+
+// Test hook (smvs_test_decode_codes): both halves of every code, decoded, and the
+// normal of a code.
+__global__ void DecodeCodesKernel(const uint32_t* __restrict__ codes, int n, float* __restrict__ quotients,
+                                  float* __restrict__ normals) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  quotients[2 * i] = Over32767(codes[i] >> 16);
+  quotients[2 * i + 1] = Over32767(codes[i] & 0x0000ffffu);
+  float v[3];
+  Decode(codes[i], v);
+  for (int k = 0; k < 3; ++k) normals[3 * i + k] = v[k];
 }
 
 __device__ __forceinline__ bool PixelOf(const CfJob& j, int local, int* col, int* row) {
@@ -964,6 +976,14 @@ void smvs_cross_filter_destroy(smvs_cross_filter* f) {
   cudaSetDevice(f->device);
   FreeAll(f);
   delete f;
+}
+
+int smvs_test_decode_codes(const uint32_t* codes, int n, float* quotients, float* normals, void* stream) {
+  if (n < 0 || (n > 0 && (!codes || !quotients || !normals))) return Fail(SMVS_EINVAL, "decode codes: bad arguments");
+  if (n == 0) return SMVS_OK;
+  DecodeCodesKernel<<<(n + 255) / 256, 256, 0, (cudaStream_t)stream>>>(codes, n, quotients, normals);
+  CF_CUDA(cudaGetLastError());
+  return SMVS_OK;
 }
 
 int smvs_cross_filter_release_cache(int gpu_index) {
