@@ -1956,8 +1956,10 @@ int EnsureScanSums(smvs_fusion* f, uint64_t n) {
   const size_t nb = (size_t)((n + kScanItems - 1) / kScanItems);
   if (nb + 1 <= f->scan_sums_cap) return SMVS_OK;
   Free(f, f->d_scan_sums);
-  f->scan_sums_cap = nb + 1;
-  return Alloc(f, &f->d_scan_sums, f->scan_sums_cap);
+  f->scan_sums_cap = 0;
+  const int st = Alloc(f, &f->d_scan_sums, nb + 1);
+  if (!st) f->scan_sums_cap = nb + 1;
+  return st;
 }
 
 // Exclusive scan of n values into out[0..n], out[n] = total.
