@@ -2270,7 +2270,7 @@ struct Carve {
   smvs_fusion* f;
   char* at;
   size_t left;
-  void* own[8] = {};
+  void* own[16] = {};
   int nown = 0;
   explicit Carve(smvs_fusion* fusion)
       : f(fusion), at(reinterpret_cast<char*>(fusion->d_pix)), left(32 * (size_t)fusion->total) {}
@@ -2320,18 +2320,30 @@ __global__ void KeepKernel(uint32_t n, const uint32_t* __restrict__ keep, const 
   for (uint32_t k = 0; k < cnt; ++k) new_vis[v + k] = vis[b + k];
 }
 
-// Keeps the points with keep[i] (1 or 0; order preserved, as the reference's
-// in-place compaction loops do). The device arrays stay where they are and only shrink.
-int Compact(smvs_fusion* f, Carve& scratch, const uint32_t* keep, size_t* removed) {
-  const uint32_t n = (uint32_t)f->num_points;
-  uint32_t *nvis, *pt_idx, *vis_idx, *new_vis = f->d_claim_cnt;
+// What Compact needs. Taken before a pass changes the cloud: a pass that runs out
+// of memory leaves it as it was.
+struct CompactScratch {
+  uint32_t *nvis, *pt_idx, *vis_idx;
   smvs_fused_point* new_pts;
   uint64_t* new_off;
+  int Take(smvs_fusion* f, Carve& scratch) {
+    const size_t n = f->num_points;
+    int st;
+    if ((st = scratch.Take(&nvis, n)) || (st = scratch.Take(&pt_idx, n + 1)) || (st = scratch.Take(&vis_idx, n + 1)) ||
+        (st = scratch.Take(&new_pts, n)) || (st = scratch.Take(&new_off, n + 1)))
+      return st;
+    return EnsureScanSums(f, n);
+  }
+};
+
+// Keeps the points with keep[i] (1 or 0; order preserved, as the reference's
+// in-place compaction loops do). The device arrays stay where they are and only shrink.
+int Compact(smvs_fusion* f, const CompactScratch& c, const uint32_t* keep, size_t* removed) {
+  const uint32_t n = (uint32_t)f->num_points;
+  uint32_t *nvis = c.nvis, *pt_idx = c.pt_idx, *vis_idx = c.vis_idx, *new_vis = f->d_claim_cnt;
+  smvs_fused_point* new_pts = c.new_pts;
+  uint64_t* new_off = c.new_off;
   int st;
-  if ((st = scratch.Take(&nvis, n)) || (st = scratch.Take(&pt_idx, (size_t)n + 1)) ||
-      (st = scratch.Take(&vis_idx, (size_t)n + 1)) || (st = scratch.Take(&new_pts, n)) ||
-      (st = scratch.Take(&new_off, (size_t)n + 1)))
-    return st;
   const int blocks = Blocks((size_t)n + 1, 256);
   KeptCountKernel<<<blocks, 256, 0, f->stream>>>(n, f->d_out_visoff, keep, nvis);
   if ((st = Scan(f, keep, n, pt_idx)) || (st = Scan(f, nvis, n, vis_idx))) return st;
@@ -3124,9 +3136,11 @@ int smvs_fusion_remove_duplicate_points(smvs_fusion* f, size_t* num_removed) {
   uint32_t *keep, *list, *counts;
   DupView* d_views;
   Carve scratch(f);
+  CompactScratch compact;
   int st;
   if ((st = scratch.Take(&keep, n)) || (st = scratch.Take(&list, n)) ||
-      (st = scratch.Take(&counts, (size_t)max_level + 1)) || (st = scratch.Take(&d_views, (size_t)f->num_views)))
+      (st = scratch.Take(&counts, (size_t)max_level + 1)) || (st = scratch.Take(&d_views, (size_t)f->num_views)) ||
+      (st = compact.Take(f, scratch)))
     return st;
   std::vector<DupView> views(f->num_views);
   for (int v = 0; v < f->num_views; ++v) {
@@ -3167,7 +3181,7 @@ int smvs_fusion_remove_duplicate_points(smvs_fusion* f, size_t* num_removed) {
   DupDropKernel<<<Blocks(n, 256), 256, 0, f->stream>>>(n, f->d_out_visoff, cells, latest, keep);
   ++f->launches;
   FU_CUDA(cudaGetLastError());
-  return Compact(f, scratch, keep, num_removed);
+  return Compact(f, compact, keep, num_removed);
 }
 
 int smvs_fusion_remove_outliers(smvs_fusion* f, int nb_neighbors, double max_spacing_factor, size_t* num_removed) {
@@ -3183,6 +3197,7 @@ int smvs_fusion_remove_outliers(smvs_fusion* f, int nb_neighbors, double max_spa
   if (n >= (1ull << 32) - 1) return Fail(SMVS_EINVAL, "fusion: too many points for the neighbour grid");
   const uint32_t nn = (uint32_t)n;
   Carve scratch(f);
+  CompactScratch compact;
   CloudStats* stats;
   uint32_t* keep;
   int st;
@@ -3234,7 +3249,8 @@ int smvs_fusion_remove_outliers(smvs_fusion* f, int nb_neighbors, double max_spa
   float4* sorted;
   float* spacing;
   if ((st = scratch.Take(&cell_of, n)) || (st = scratch.Take(&counts, cells)) ||
-      (st = scratch.Take(&startv, cells + 1)) || (st = scratch.Take(&sorted, n)) || (st = scratch.Take(&spacing, n)))
+      (st = scratch.Take(&startv, cells + 1)) || (st = scratch.Take(&sorted, n)) || (st = scratch.Take(&spacing, n)) ||
+      (st = compact.Take(f, scratch)))
     return st;
   const int K = nb_neighbors + 1;
   FU_CUDA(cudaMemsetAsync(counts, 0, cells * sizeof(uint32_t), f->stream));
@@ -3275,7 +3291,7 @@ int smvs_fusion_remove_outliers(smvs_fusion* f, int nb_neighbors, double max_spa
   BinKeepKernel<<<Blocks(n, 256), 256, 0, f->stream>>>(f->d_out_pts, nn, stats, mask, keep);
   ++f->launches;
   FU_CUDA(cudaGetLastError());
-  return Compact(f, scratch, keep, num_removed);
+  return Compact(f, compact, keep, num_removed);
 }
 
 void smvs_fusion_destroy(smvs_fusion* f) {

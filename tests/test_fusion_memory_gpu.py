@@ -106,3 +106,56 @@ def test_clean_up_can_be_called_again_after_it_ran_out_of_memory(call):
                 got = getattr(f, call)()
             assert got <= points and len(f.GetFusedPoints()) == points - got
     assert failures < 15 and (failures > 0 or call == "RemoveDuplicatePoints")
+
+
+@pytest.mark.parametrize("call", ["RemoveOutliers", "RemoveDuplicatePoints"])
+def test_clean_up_that_runs_out_of_memory_leaves_the_cloud(call):
+    """Two images from one place: a point for nearly every pixel pair, so that the
+    clean-up does not fit into the image loop's arrays. Whichever allocation fails,
+    points, scores and images stay as they were, and the next call gives what the
+    first would have."""
+    images, _ = _inputs()
+    options = FusionOptions(min_num_pixels=2, max_num_pixels=2, min_num_visible_images=1, max_normal_error=90.0,
+                            max_depth_error=0.1)
+    keep = [images[0], images[0]]
+    lists = [[1], [0]]
+
+    def cloud(f):
+        return [a.copy().view(np.uint8) for a in (f.GetFusedPoints(), *f.VisibilityCSR())]
+
+    def same(a, b):
+        for x, y in zip(a, b):
+            np.testing.assert_array_equal(x, y)
+
+    def fusion():  # without the projection table, which would make room
+        N.check(N.lib().smvs_test_fusion_paths(1, 0))
+        try:
+            return StereoFusion(options, keep, lists)
+        finally:
+            N.check(N.lib().smvs_test_fusion_paths(0, 0))
+
+    with fusion() as f:
+        f.Run()
+        assert len(f.GetFusedPoints()) > 3 * keep[0].depth.size // 4
+        before = cloud(f)
+        dropped = getattr(f, call)()
+        after = cloud(f)
+    failures = 0
+    for nth in range(1, 16):
+        with fusion() as f:
+            f.Run()
+            N.check(N.lib().smvs_test_fail_allocation(nth))
+            try:
+                got = getattr(f, call)()
+            except N.SmvsError as error:
+                assert error.status == N.SMVS_ENOMEM
+                got = None
+            finally:
+                N.check(N.lib().smvs_test_fail_allocation(0))
+            if got is None:
+                failures += 1
+                same(cloud(f), before)
+                got = getattr(f, call)()
+            assert got == dropped
+            same(cloud(f), after)
+    assert failures < 15 and (failures > 0 or call == "RemoveDuplicatePoints")
