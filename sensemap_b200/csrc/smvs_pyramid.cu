@@ -258,6 +258,13 @@ int smvs_resample_maps(const float* depth, const float* normal, int width, int h
       out_width <= 0 || out_height <= 0)
     return Fail(SMVS_EINVAL, "smvs_resample_maps: bad arguments");
   cudaStream_t s = (cudaStream_t)stream;
+  // Normals that go where the depth map lies wait until it has been read.
+  const char *n0 = reinterpret_cast<const char*>(out_normal), *d0 = reinterpret_cast<const char*>(depth);
+  if (depth && normal && d0 < n0 + 12 * (size_t)out_width * out_height && n0 < d0 + 4 * (size_t)width * height) {
+    const int st = smvs_resample_maps(depth, nullptr, width, height, out_depth, nullptr, out_width, out_height, stream);
+    return st ? st
+              : smvs_resample_maps(nullptr, normal, width, height, nullptr, out_normal, out_width, out_height, stream);
+  }
   // Rows share their input only where the map grows: 1500x1000 to 3000x2000 takes
   // 42 us with four rows a thread, 58 with one; the way back 36 and 30 (cold L2).
   if (out_height <= height)
