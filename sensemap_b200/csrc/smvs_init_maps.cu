@@ -790,6 +790,21 @@ int Outputs(Call* call, const smvs_view* view, float* depth, float* normal, floa
   return st;
 }
 
+// The points are read while the maps are written: an input on the device that the
+// output maps overlap is copied first.
+int Apart(Call* call, const float** in, size_t count, const float* depth, const float* normal, size_t wh) {
+  if (call->memory != SMVS_MEM_DEVICE || count == 0) return SMVS_OK;
+  const float* p = *in;
+  auto meets = [&](const float* map, size_t n) { return p < map + n && map < p + count; };
+  if (!meets(depth, wh) && !meets(normal, 3 * wh)) return SMVS_OK;
+  float* copy;
+  const int st = call->Alloc(&copy, count * sizeof(float));
+  if (st) return st;
+  IM_CUDA(cudaMemcpyAsync(copy, p, count * sizeof(float), cudaMemcpyDeviceToDevice, call->stream));
+  *in = copy;
+  return SMVS_OK;
+}
+
 // `words` 32-bit words of scratch, all ones, and the call's status.
 int Scratch(Call* call, size_t words, uint32_t** p, Status** status) {
   int st = call->Alloc(p, words * 4);
@@ -959,6 +974,9 @@ int smvs_init_depth_from_dense_points(const smvs_view* view, const float* xyz, c
   PixelState s;
   Status* status;
   if ((st = call.In(xyz, num_points * 3, &d_xyz)) || (st = call.In(normals, num_points * 3, &d_n))) return st;
+  if ((st = Apart(&call, &d_xyz, num_points * 3, depth, normal, wh)) ||
+      (st = Apart(&call, &d_n, num_points * 3, depth, normal, wh)))
+    return st;
   if ((st = Outputs(&call, view, depth, normal, &d_depth, &d_normal))) return st;
   if ((st = PixelScratch(&call, (size_t)(view->width / 2) * (view->height / 2), &s, &status))) return st;
   const Cam c = MakeCam(*view);
