@@ -44,7 +44,7 @@ CPU_BAND_ROWS = 16         # rows of the CPU oracle's band sample (both passes)
 # DRAM bytes (read + write) of one sweep launch of the bench workload per source
 # storage, from ncu (dram__bytes_read.sum + dram__bytes_write.sum of one
 # SweepKernelL<5,1,12> launch, profiles/sweep_kernel_1600x1200_n10_f16.md).
-SWEEP_DRAM_BYTES: dict = {"f16": 0.548e9 + 0.587e9}
+SWEEP_DRAM_BYTES: dict = {"f16": 0.391e9 + 0.504e9}
 
 
 def log(*a):

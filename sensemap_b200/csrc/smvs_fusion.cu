@@ -2848,7 +2848,7 @@ int smvs_fusion_create(const smvs_fusion_options* opt, const smvs_fusion_view* v
   // its point in the image and in each overlapping image (about 16 each for
   // the default 2 pixels), each with one push per overlapping image. Start the
   // pool at that bound for the largest image (within a quarter of the free
-  // device memory); it grows if an image needs more.
+  // device memory, but at least 64 words a pixel); it grows if an image needs more.
   int max_deg = 0;
   for (int v = 0; v < num_views; ++v) {
     max_deg = std::max(max_deg, overlap_offsets[v + 1] - overlap_offsets[v]);

@@ -167,8 +167,8 @@ __device__ __forceinline__ void FoldRange(uint32_t lo, uint32_t hi, Status* st) 
 // after another, a lane a pixel: neighbouring lanes touch neighbouring pixels. A
 // stored key only ever falls, so one that is not above the point's needs no atomic;
 // the read costs less than the atomic that it saves. Bound by the latency of the
-// L2; 400,000 points into 1600x1200 (49 pixels each): 47 us, the whole call 126 us
-// (201 us with a thread and 49 atomics a point).
+// L2; 400,000 points into 1600x1200 (49 pixels each): 47 us, the whole call, waited
+// for, 126 us on the host's clock (201 us with a thread and 49 atomics a point).
 __global__ void __launch_bounds__(kThreads) SparseSplatKernel(Cam c, const float* __restrict__ xyz, size_t n,
                                                               int per, uint32_t* __restrict__ key,
                                                               Status* __restrict__ st) {
@@ -363,10 +363,10 @@ __device__ __forceinline__ bool FaceDepth(const FaceRec& r, const double* Kinv, 
 // visit(record, index, x, y) for the pixels of every record's box [u0, u1] x [v0, v1]
 // (none where u0 > u1): by the record's thread while the box is small, by the whole
 // warp, a lane a pixel, from kWarpBox pixels on. `per` records a warp. 1600x1200,
-// whole call: a mesh of 400,000 small faces 246 us (379 us with a thread a face and
-// two passes), one of 4,000 faces with 31x31 boxes 145 us (829 us). Delaunay planes of
-// 2,000 points in 1600x1066: the two kernels 0.58 + 1.98 ms with a thread a triangle,
-// now 0.03 + 0.10 ms.
+// whole call, waited for, on the host's clock: a mesh of 400,000 small faces 246 us
+// (379 us with a thread a face and two passes), one of 4,000 faces with 31x31 boxes
+// 145 us (829 us). Delaunay planes of 2,000 points in 1600x1066: the two kernels
+// 0.58 + 1.98 ms with a thread a triangle, now 0.03 + 0.10 ms.
 constexpr int kWarpBox = 32;
 
 template <typename Rec, typename Visit>
@@ -471,9 +471,9 @@ __device__ __forceinline__ bool Window(const Cam& c, const float* __restrict__ x
 // any window: a warp, in several steps). `per` points a group, at most kGroup: fewer
 // where the points are too few to fill the GPU. 400,000 points into 1600x1200 with
 // ws 4, 25 slots each: 47 us, bound by the latency of its accesses to the L2 (64
-// registers for four windows in flight; 40, or fewer windows, took longer); the two passes of a
-// thread a point, two atomics a slot in the first, took 178 us, and the whole call
-// 358 us, now 126 us.
+// registers for four windows in flight; 40, or fewer windows, took longer); the two
+// passes of a thread a point, two atomics a slot in the first, took 178 us, and the
+// whole call, among others on the stream, 326 us, now 106 us.
 template <int kGroup, int kSide>
 __global__ void __launch_bounds__(kThreads) PointScatterKernel(Cam c, const float* __restrict__ xyz,
                                                                const float* __restrict__ nrm, size_t n, int ws,

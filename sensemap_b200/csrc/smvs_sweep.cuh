@@ -209,6 +209,9 @@ __device__ __forceinline__ float CombineClasses(const float* a, unsigned gmask) 
 // it shortens the init-conf and local-optimisation launches by 11 % and 8 % and
 // lengthens the sweep's by 1 %, so those two kernels ask for it. The
 // arithmetic and its order do not change.
+// TapWeight and WindowCost (smvs_spread.cuh) spell out the roundings that the
+// compiler chooses here; test_spread_gpu compares every instance, and UseSpread leaves
+// out the one that is compiled with others.
 template <int R, int S, int G, bool kUnrollRows = false>
 __device__ __forceinline__ float NccCost(cudaTextureObject_t tex, const float* pose, int row, int col, float depth,
                                          const float n[3], const float iK[4], int W, int H, float center,
