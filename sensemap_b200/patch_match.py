@@ -134,9 +134,10 @@ def _is_cuda_tensor(x) -> bool:
 
 def _sync_producers(keep, stream) -> None:
     """The library reads device inputs on its own stream: when no stream is
-    given, wait for the torch stream that produced them (and for any
-    contiguous() copy made here) before handing their addresses over."""
-    if stream is None and any(_is_cuda_tensor(o) for o in keep if o is not None):
+    given (0, the default stream's handle, reads as none), wait for the torch
+    stream that produced them (and for any contiguous() copy made here) before
+    handing their addresses over."""
+    if not stream and any(_is_cuda_tensor(o) for o in keep if o is not None):
         import torch
         torch.cuda.current_stream().synchronize()
 
@@ -340,6 +341,7 @@ def autotune(options: PatchMatchOptions, problem: Problem, stream=None, repeats:
     """Launch-shape autotuner (smvs_autotune): the fastest sweep launch shape for
     this problem, with every candidate's ms per sweep launch."""
     prob, keep = _problem_struct(problem)
+    _sync_producers(keep, stream)
     best = N.smvs_tuning()
     cap = 32
     tried = (N.smvs_tuning * cap)()

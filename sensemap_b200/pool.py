@@ -13,7 +13,15 @@ import ctypes as C
 import numpy as np
 
 from . import _native as N
-from .patch_match import PatchMatchOptions, View, _addr, _is_cuda_tensor
+from .patch_match import PatchMatchOptions, View, _addr, _is_cuda_tensor, _sync_producers
+
+
+def _wait_for_copies(pairs) -> None:
+    """The pool reads device inputs after the call: a copy made here (a dtype or
+    layout that it does not take) must not go back to torch before that."""
+    if any(_is_cuda_tensor(used) and used is not given for used, given in pairs if used is not None):
+        import torch
+        torch.cuda.synchronize()
 
 
 class DepthMapPool:
@@ -35,6 +43,7 @@ class DepthMapPool:
         N.check(N.lib().smvs_pool_create(C.byref(o), C.c_void_p(int(stream)) if stream is not None else None,
                                          C.byref(h)))
         self._h = h
+        self._stream = int(stream) if stream else None
         self._shapes = {}   # view id -> (H, W)
         self._jobs = {}     # job id -> (H, W, N)
 
@@ -57,9 +66,10 @@ class DepthMapPool:
         cv.R[:] = [float(a) for a in np.asarray(view.R, np.float64).reshape(9)]
         cv.T[:] = [float(a) for a in np.asarray(view.T, np.float64).reshape(3)]
         cv.scale = 1.0
+        _sync_producers([keep], self._stream)
         N.check(N.lib().smvs_pool_add_view(self._h, int(view_id), C.byref(cv), N.MEM_DEVICE if dev else N.MEM_HOST))
         self._shapes[int(view_id)] = (view.height, view.width)
-        del keep
+        _wait_for_copies([(keep, view.image)])
 
     def has_view(self, view_id: int) -> bool:
         r = C.c_int()
@@ -70,8 +80,9 @@ class DepthMapPool:
         dp, dk, ddev = _addr(depth if _is_cuda_tensor(depth) else np.asarray(depth, np.float32))
         np_, nk, _ = _addr(None if normal is None else (normal if _is_cuda_tensor(normal)
                                                         else np.asarray(normal, np.float32)))
+        _sync_producers([dk, nk], self._stream)
         N.check(N.lib().smvs_pool_set_view_maps(self._h, int(view_id), dp, np_, N.MEM_DEVICE if ddev else N.MEM_HOST))
-        del dk, nk
+        _wait_for_copies([(dk, depth), (nk, normal)])
 
     def submit(self, options: PatchMatchOptions, ref_view: int, src_views) -> int:
         srcs = (C.c_int64 * len(src_views))(*[int(s) for s in src_views])
