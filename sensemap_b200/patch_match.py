@@ -13,6 +13,7 @@ from __future__ import annotations
 
 import ctypes as C
 import math
+import weakref
 from dataclasses import dataclass, field, fields
 from typing import Optional, Sequence
 
@@ -113,10 +114,12 @@ class Problem:
 class DeviceBuffer:
     """A raw device pointer (e.g. another engine's map from DeviceMaps()) with
     its shape, usable wherever a View takes an array. The owner must outlive
-    every engine that reads it."""
+    every engine that reads it; an engine given as `owner` has finished its
+    work before another stream reads the map."""
 
-    def __init__(self, ptr: int, shape, dtype=np.float32):
+    def __init__(self, ptr: int, shape, dtype=np.float32, owner=None):
         self.ptr = int(ptr)
+        self.owner = weakref.ref(owner) if owner is not None else None
         self.shape = tuple(shape)
         self.dtype = np.dtype(dtype)
         self.is_cuda = True
@@ -136,8 +139,14 @@ def _sync_producers(keep, stream) -> None:
     """The library reads device inputs on its own stream: when no stream is
     given (0, the default stream's handle, reads as none), wait for the torch
     stream that produced them (and for any contiguous() copy made here) before
-    handing their addresses over."""
-    if not stream and any(_is_cuda_tensor(o) for o in keep if o is not None):
+    handing their addresses over. Maps of an engine on another stream wait for
+    that engine."""
+    device = [o for o in keep if o is not None and _is_cuda_tensor(o)]
+    owners = {id(e): e for e in (o.owner() for o in device if getattr(o, "owner", None) is not None) if e is not None}
+    for engine in owners.values():
+        if engine._h is not None and (not stream or engine._stream != int(stream)):
+            engine.Synchronize()
+    if not stream and device:
         import torch
         torch.cuda.current_stream().synchronize()
 
@@ -234,6 +243,7 @@ class PatchMatchACMMCuda:
         stream_ptr = C.c_void_p(int(stream)) if stream is not None else None
         N.check(lib.smvs_create(C.byref(options.to_c()), C.byref(prob), stream_ptr, C.byref(handle)))
         self._h = handle
+        self._stream = int(stream) if stream else None
         self._keep = keep  # device inputs must outlive the engine's queued copies
         self.width = problem.images[problem.ref_image_idx].width
         self.height = problem.images[problem.ref_image_idx].height
@@ -287,8 +297,8 @@ class PatchMatchACMMCuda:
     def DeviceDepthNormal(self):
         """(depth, normal) as DeviceBuffers over this engine's maps (valid until close())."""
         m = self.DeviceMaps()
-        return (DeviceBuffer(m.depth, (self.height, self.width)),
-                DeviceBuffer(m.normal, (3, self.height, self.width)))
+        return (DeviceBuffer(m.depth, (self.height, self.width), owner=self),
+                DeviceBuffer(m.normal, (3, self.height, self.width), owner=self))
 
     def LaunchCount(self) -> int:
         return int(N.lib().smvs_launch_count(self._h))

@@ -141,7 +141,6 @@ class PyramidPatchMatch:
                     passes += 1
                 peak = max(peak, self._device_used())
                 maps = {r: pm.DeviceDepthNormal() for r, pm in photo.items()}
-                maps = {r: (_as_tensor(d), _as_tensor(n)) for r, (d, n) in maps.items()}
                 geo = {}
                 for r in self.problems:
                     pm = self._pass(replace(self.options, geom_consistency=True, init_depth_random=False), r,
