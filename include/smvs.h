@@ -164,8 +164,10 @@ typedef struct smvs_engine smvs_engine;
 
 /* Device pointers to an engine's maps (valid until smvs_destroy). Each is a
  * cudaMalloc allocation of its own: other streams, peer devices and, through
- * cudaIpcGetMemHandle, other processes may read it. Layouts are dense row-major; normal and cost are planar (slice-major), like GpuMat's
- * slices (src/util/gpu_mat.h:194-198) without the pitch. */
+ * cudaIpcGetMemHandle, other processes may read it, after smvs_synchronize where
+ * they do not run on the engine's stream. Layouts are dense row-major; normal and
+ * cost are planar (slice-major), like GpuMat's slices (src/util/gpu_mat.h:194-198)
+ * without the pitch. */
 typedef struct smvs_device_maps {
   int width, height, num_src;
   float* depth;      /* W*H */
